@@ -11,12 +11,17 @@
 #include "fdp_host.h"
 #include "fdp_launch.h"
 #include "fdp_rowinit_dev.h"
+#include "fdp_tail_dev.h"
 
 using fdp::DevTables;
 
 static thread_local std::string g_last_error;
 
 #define FDP_RUN_MAX_MODULI 64
+
+// Device memory left free beside an escape buffer.
+static constexpr size_t kEscapeMargin = size_t(1) << 30;
+static constexpr size_t kWindowEscapes = size_t(1) << 30;
 
 static fdp_status cuda_status(cudaError_t e, const char *what) {
   if (e == cudaSuccess) return FDP_OK;
@@ -153,6 +158,7 @@ fdp_ctx::~fdp_ctx() {
   for (auto &kv : tables) fdp::free_tables(&kv.second);
   if (d_main) cudaFree(d_main);
   if (d_blk) cudaFree(d_blk);
+  if (d_esc) cudaFree(d_esc);
   if (d_acc) cudaFree(d_acc);
   if (d_res) cudaFree(d_res);
   if (h_res) cudaFreeHost(h_res);
@@ -162,6 +168,7 @@ fdp_ctx::~fdp_ctx() {
   if (ev1) cudaEventDestroy(ev1);
   if (span_fork) cudaEventDestroy(span_fork);
   if (span_join) cudaEventDestroy(span_join);
+  if (esc_pool) cudaMemPoolDestroy(esc_pool);
   if (span_stream) cudaStreamDestroy(span_stream);
   if (stream) cudaStreamDestroy(stream);
 }
@@ -215,6 +222,7 @@ fdp_status fdp_prepare_pass(fdp_ctx *c, int W, const DevTables **full) {
   if (s != FDP_OK) return s;
   int rcap = 0;
   if (const int R = row_init_rows(c, W, &rcap)) FDP_CK(fdp::prepare_row_init(W, R, rcap), "row-k initialiser tables");
+  if (c->cfg.tail) FDP_CK(fdp::prepare_tail(W), "row tail tables");
   if (!c->cfg.bounded_prefix || W < 4) return s;
   std::vector<int> caps = fdp::bounded_prefix_caps(W);
   caps.push_back(1);
@@ -233,6 +241,30 @@ static fdp_status ensure_buffer(uint32_t **buf, size_t *cap, size_t bytes, const
   *cap = 0;
   FDP_CK(cudaMalloc(buf, bytes ? bytes : 4), what);
   *cap = bytes;
+  return FDP_OK;
+}
+
+// The context's state buffers for `lanes` lanes of width W, and, where
+// `want_esc` and device memory allow, the escape words of the fused row tail.
+// Those are optional: they go first when a state buffer has to grow, and a
+// pass without them runs every cell as its own launch.
+static fdp_status ensure_state(fdp_ctx *c, int W, int lanes, bool want_esc) {
+  const size_t mb = size_t(fdp::main_states(W)) * lanes * 4, bb = size_t(fdp::blocked_states(W)) * lanes * 4;
+  const size_t eb = want_esc ? size_t(fdp::tail_escape_words(W)) * lanes * 4 : 0;
+  if (c->d_esc && (c->cap_main < mb || c->cap_blk < bb || c->cap_esc < eb)) {
+    cudaFree(c->d_esc);
+    c->d_esc = nullptr;
+    c->cap_esc = 0;
+  }
+  fdp_status s = ensure_buffer(&c->d_main, &c->cap_main, mb, "main state");
+  if (s == FDP_OK) s = ensure_buffer(&c->d_blk, &c->cap_blk, bb, "blocked state");
+  if (s != FDP_OK || !eb || c->cap_esc >= eb) return s;
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b > eb + kEscapeMargin &&
+      cudaMalloc(&c->d_esc, eb) == cudaSuccess)
+    c->cap_esc = eb;
+  else
+    cudaGetLastError();
   return FDP_OK;
 }
 
@@ -265,7 +297,7 @@ extern "C" fdp_status fdp_test_inject_pass_errors(int count) {
 }
 
 fdp_status fdp_enqueue_pass(fdp_ctx *c, const DevTables &t, int L, const uint32_t *mods, uint32_t *main,
-                            uint32_t *blk, unsigned long long *acc, uint32_t *d_res, uint32_t *h_res,
+                            uint32_t *blk, uint32_t *esc, unsigned long long *acc, uint32_t *d_res, uint32_t *h_res,
                             unsigned int *d_err, cudaStream_t s, uint64_t *launches, cudaStream_t span_stream,
                             cudaEvent_t fork, cudaEvent_t join) {
   const int W = t.W;
@@ -316,7 +348,21 @@ fdp_status fdp_enqueue_pass(fdp_ctx *c, const DevTables &t, int L, const uint32_
   }
   if (prev != &t) FDP_CK(fdp::enqueue_expand(*prev, t, L, main, blk, D * uint64_t(L), s, &n), "grow state");
   const int row0 = next_row > B + 1 ? next_row : B + 1;
-  const bool chains = span_stream && fork && join && c->cfg.span_chains && L > 8 && !c->cfg.split_panels &&
+  const bool fused = esc && c->cfg.tail && fdp::tail_symbols(W);
+  // One row in the full space: its cells one launch each, or, given escape
+  // words, cells s-1..1 as one fused pass.
+  auto full_row = [&](int lanes, const uint32_t *m, uint32_t *mn, uint32_t *bk, uint32_t *es,
+                      cudaStream_t ss) -> fdp_status {
+    const int last = fused ? fdp::tail_symbols(W) : 1;
+    for (int p = W - 1; p >= last; --p)
+      FDP_CK(fdp::launch_cell(t, lanes, m, mn, bk, p, p == W - 1, false, c->cfg, ss, &n), "cell");
+    if (last > 1) FDP_CK(fdp::launch_tail(t, lanes, m, mn, bk, es, ss, &n), "row tail");
+    return FDP_OK;
+  };
+  // Span chains overlap the tails of single-cell launches; with the fused row
+  // tail one chain is faster (n = 20, 14 lanes: 1.40 against 1.53 s), as its CTAs
+  // take whole SMs and hold back the other chain's.
+  const bool chains = !fused && span_stream && fork && join && c->cfg.span_chains && L > 8 && !c->cfg.split_panels &&
                       c->cfg.split_spans_min_p <= 1 && row0 <= fdp::sweep_rows(W);
   if (chains) {
     // Each lane span is laid out as a lane count of its own at its first
@@ -328,19 +374,16 @@ fdp_status fdp_enqueue_pass(fdp_ctx *c, const DevTables &t, int L, const uint32_
       const int le = fdp::span_end_of(L, l0);
       cudaStream_t ss = i == 0 ? s : span_stream;
       for (int row = row0; row <= fdp::sweep_rows(W); ++row)
-        for (int p = W - 1; p >= 1; --p)
-          FDP_CK(fdp::launch_cell(t, le - l0, mods + l0, main + size_t(l0) * M, blk + size_t(l0) * D, p, p == W - 1,
-                                  false, c->cfg, ss, &n),
-                 "cell");
+        if ((st = full_row(le - l0, mods + l0, main + size_t(l0) * M, blk + size_t(l0) * D,
+                           esc ? esc + size_t(l0) * fdp::tail_escape_words(W) : nullptr, ss)) != FDP_OK)
+          return st;
       l0 = le;
     }
     FDP_CK(cudaEventRecord(join, span_stream), "span join");
     FDP_CK(cudaStreamWaitEvent(s, join, 0), "span join");
   } else {
     for (int row = row0; row <= fdp::sweep_rows(W); ++row)
-      for (int p = W - 1; p >= 1; --p) {
-        FDP_CK(fdp::launch_cell(t, L, mods, main, blk, p, p == W - 1, false, c->cfg, s, &n), "cell");
-      }
+      if ((st = full_row(L, mods, main, blk, esc, s)) != FDP_OK) return st;
   }
   FDP_CK(fdp::launch_first_row_dot(t, L, mods, main, acc, d_res, s), "first-row dot");
   n += 2;
@@ -364,9 +407,7 @@ extern "C" fdp_status fdp_run_sync(fdp_ctx *c, const fdp_problem *pr, uint32_t *
   const DevTables *t = nullptr;
   if ((s = fdp_prepare_pass(c, W, &t)) != FDP_OK) return s;
   const int lanes = pr->lanes < pr->k ? pr->lanes : pr->k;
-  const uint64_t M = fdp::main_states(W), D = fdp::blocked_states(W);
-  if ((s = ensure_buffer(&c->d_main, &c->cap_main, size_t(M) * lanes * 4, "main state")) != FDP_OK) return s;
-  if ((s = ensure_buffer(&c->d_blk, &c->cap_blk, size_t(D) * lanes * 4, "blocked state")) != FDP_OK) return s;
+  if ((s = ensure_state(c, W, lanes, c->cfg.tail)) != FDP_OK) return s;
   // Every pass (lanes residues each) is captured into ONE graph, run with one launch.
   fdp_run_stats acc{};
   auto c0 = std::chrono::steady_clock::now();
@@ -377,7 +418,7 @@ extern "C" fdp_status fdp_run_sync(fdp_ctx *c, const fdp_problem *pr, uint32_t *
   fdp_status es = cuda_status(fdp_enqueue_err_reset(c->d_err, c->stream), "error word");
   for (int done = 0; done < pr->k && es == FDP_OK; done += lanes) {
     const int L = (pr->k - done) < lanes ? (pr->k - done) : lanes;
-    es = fdp_enqueue_pass(c, *t, L, pr->moduli + done, c->d_main, c->d_blk, c->d_acc, c->d_res, c->h_res + done,
+    es = fdp_enqueue_pass(c, *t, L, pr->moduli + done, c->d_main, c->d_blk, c->d_esc, c->d_acc, c->d_res, c->h_res + done,
                           c->d_err, c->stream, &launches, c->span_stream, c->span_fork, c->span_join);
   }
   if (es == FDP_OK) es = cuda_status(fdp_enqueue_err_read(c->h_err, c->d_err, c->stream), "error word");
@@ -416,6 +457,39 @@ extern "C" fdp_status fdp_run_sync(fdp_ctx *c, const fdp_problem *pr, uint32_t *
   return FDP_OK;
 }
 
+// Escape words for one window of fdp_apply_cells, or null: allocated and freed
+// in the order of the caller's stream, so windows on other streams get words of
+// their own.  The pool is the context's and keeps kWindowEscapes bytes between
+// calls; a window that needs more runs cell by cell, as mapping fresh memory
+// for each call costs more than the fused tail gives (15.7 GB at width 24, one
+// lane: a first window 1387 against 857 ms).  So does a stream under capture
+// (the captured work must not depend on an allocation of this context).
+static uint32_t *window_escapes(fdp_ctx *c, int W, int lanes, cudaStream_t st) {
+  const size_t bytes = size_t(fdp::tail_escape_words(W)) * lanes * 4;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (!bytes || bytes > kWindowEscapes || !c->cfg.tail || cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  uint32_t *p = nullptr;
+  bool ok = fdp::prepare_tail(W) == cudaSuccess;
+  if (ok && !c->esc_pool) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = c->device;
+    uint64_t keep = kWindowEscapes;
+    ok = cudaMemPoolCreate(&c->esc_pool, &props) == cudaSuccess;
+    if (ok) cudaMemPoolSetAttribute(c->esc_pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    else c->esc_pool = nullptr;
+  }
+  if (!ok || cudaMallocFromPoolAsync(&p, bytes, c->esc_pool, st) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  return p;
+}
+
 extern "C" fdp_status fdp_apply_cells(fdp_ctx *c, int width, int p_hi, int p_lo, int lanes, const uint32_t *moduli,
                                       uint32_t *d_main, uint32_t *d_block, void *stream) {
   // Checked first, before anything that needs a context or a device.
@@ -438,8 +512,20 @@ extern "C" fdp_status fdp_apply_cells(fdp_ctx *c, int width, int p_hi, int p_lo,
   fdp_status s = fdp_ctx_tables(c, width, &t);
   if (s != FDP_OK) return s;
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : c->stream;
-  for (int p = p_hi; p >= p_lo; --p)
-    FDP_CK(fdp::launch_cell(*t, lanes, moduli, d_main, d_block, p, false, true, c->cfg, st), "cell");
+  // A window that reaches down to cell 1 runs its low cells as one fused pass
+  // where the escape words can be had.
+  uint32_t *esc = p_lo == 1 && p_hi >= fdp::tail_symbols(width) - 1 ? window_escapes(c, width, lanes, st) : nullptr;
+  const int last = esc ? fdp::tail_symbols(width) : p_lo;
+  cudaError_t e = cudaSuccess;
+  for (int p = p_hi; p >= last && e == cudaSuccess; --p)
+    e = fdp::launch_cell(*t, lanes, moduli, d_main, d_block, p, false, true, c->cfg, st);
+  if (esc) {
+    if (e == cudaSuccess) e = fdp::launch_tail(*t, lanes, moduli, d_main, d_block, esc, st, nullptr);
+    if (e == cudaSuccess) e = cudaMemsetAsync(d_block, 0, size_t(fdp::blocked_states(width)) * lanes * 4, st);
+    const cudaError_t fe = cudaFreeAsync(esc, st);
+    if (e == cudaSuccess) e = fe;
+  }
+  FDP_CK(e, "cell");
   return FDP_OK;
 }
 
@@ -491,9 +577,7 @@ extern "C" fdp_status fdp_time_cells(fdp_ctx *c, const fdp_problem *pr, int rows
   const DevTables *t = nullptr;
   if ((s = fdp_ctx_tables(c, W, &t)) != FDP_OK) return s;
   const int L = pr->lanes < pr->k ? pr->lanes : pr->k;
-  const uint64_t M = fdp::main_states(W), D = fdp::blocked_states(W);
-  if ((s = ensure_buffer(&c->d_main, &c->cap_main, size_t(M) * L * 4, "main state")) != FDP_OK) return s;
-  if ((s = ensure_buffer(&c->d_blk, &c->cap_blk, size_t(D) * L * 4, "blocked state")) != FDP_OK) return s;
+  if ((s = ensure_state(c, W, L, false)) != FDP_OK) return s;
   std::vector<cudaEvent_t> ev(size_t(rows) * W * 2);
   for (auto &e : ev) FDP_CK(cudaEventCreate(&e), "event");
   // One untimed launch first: the first launch of a kernel variant also loads
@@ -580,7 +664,7 @@ extern "C" fdp_status fdp_get_tuning(fdp_ctx *c, fdp_tuning *t) {
 struct MultiPart {
   const DevTables *t = nullptr;
   int lanes = 1;
-  uint32_t *main = nullptr, *blk = nullptr, *res = nullptr;
+  uint32_t *main = nullptr, *blk = nullptr, *esc = nullptr, *res = nullptr;
   unsigned long long *acc = nullptr;
   unsigned int *err = nullptr;  // this problem's error word
   cudaStream_t s = nullptr;
@@ -615,6 +699,7 @@ extern "C" fdp_status fdp_run_multi_sync(fdp_ctx *c, const fdp_problem *probs, i
       MultiPart &p = parts[i];
       if (p.main) cudaFree(p.main);
       if (p.blk) cudaFree(p.blk);
+      if (p.esc) cudaFree(p.esc);
       if (p.acc) cudaFree(p.acc);
       if (p.res) cudaFree(p.res);
       if (p.err) cudaFree(p.err);
@@ -642,6 +727,13 @@ extern "C" fdp_status fdp_run_multi_sync(fdp_ctx *c, const fdp_problem *probs, i
     p.lanes = probs[i].lanes < probs[i].k ? probs[i].lanes : probs[i].k;
     MULTI_CK(cudaMalloc(&p.main, size_t(fdp::main_states(W)) * p.lanes * 4), "multi main state");
     MULTI_CK(cudaMalloc(&p.blk, size_t(fdp::blocked_states(W)) * p.lanes * 4 + 4), "multi blocked state");
+    const size_t eb = c->cfg.tail ? size_t(fdp::tail_escape_words(W)) * p.lanes * 4 : 0;
+    size_t free_b = 0, total_b = 0;
+    if (eb && (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b < eb + kEscapeMargin ||
+               cudaMalloc(&p.esc, eb) != cudaSuccess)) {
+      cudaGetLastError();
+      p.esc = nullptr;
+    }
     MULTI_CK(cudaMalloc(&p.acc, sizeof(unsigned long long) * FDP_MAX_LANES), "multi acc");
     MULTI_CK(cudaMalloc(&p.res, sizeof(uint32_t) * FDP_MAX_LANES), "multi res");
     MULTI_CK(cudaMalloc(&p.err, sizeof(unsigned int)), "multi error word");
@@ -663,7 +755,7 @@ extern "C" fdp_status fdp_run_multi_sync(fdp_ctx *c, const fdp_problem *probs, i
     rs = cuda_status(fdp_enqueue_err_reset(p.err, p.s), "error word");
     for (int done = 0; done < probs[i].k && rs == FDP_OK; done += p.lanes) {
       const int L = (probs[i].k - done) < p.lanes ? (probs[i].k - done) : p.lanes;
-      rs = fdp_enqueue_pass(c, *p.t, L, probs[i].moduli + done, p.main, p.blk, p.acc, p.res, pinned + off + done,
+      rs = fdp_enqueue_pass(c, *p.t, L, probs[i].moduli + done, p.main, p.blk, p.esc, p.acc, p.res, pinned + off + done,
                             p.err, p.s, &launches, p.span_s, p.span_fork, p.span_join);
     }
     if (rs == FDP_OK)

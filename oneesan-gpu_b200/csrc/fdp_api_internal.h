@@ -14,7 +14,9 @@ struct fdp_ctx {
   std::map<int, fdp::DevTables> tables;  // per frontier width
   uint32_t *d_main = nullptr;            // run_sync state, [M][lanes]
   uint32_t *d_blk = nullptr;             // run_sync state, [D][lanes]
-  size_t cap_main = 0, cap_blk = 0;
+  uint32_t *d_esc = nullptr;             // escape words of the fused row tail (optional)
+  size_t cap_main = 0, cap_blk = 0, cap_esc = 0;
+  cudaMemPool_t esc_pool = nullptr;      // escape words of fdp_apply_cells, stream-ordered
   unsigned long long *d_acc = nullptr;   // first-row dot accumulators
   uint32_t *d_res = nullptr;             // residues on the device
   uint32_t *h_res = nullptr;             // residues, pinned host
@@ -35,11 +37,12 @@ struct fdp_ctx {
 fdp_status fdp_ctx_tables(fdp_ctx *c, int W, const fdp::DevTables **out);
 fdp_status fdp_ctx_tables_cap(fdp_ctx *c, int W, int cap, const fdp::DevTables **out);
 fdp_status fdp_prepare_pass(fdp_ctx *c, int W, const fdp::DevTables **full);
-// One residue pass of L lanes on stream s.  With span_stream (and fork /
+// One residue pass of L lanes on stream s.  esc: fdp::tail_escape_words(W) x L
+// words for the fused row tail, or null to run every cell as its own launch.  With span_stream (and fork /
 // join events) given, a pass of more than 8 lanes sweeps its second lane span
 // on that stream, concurrently with the first on s.
 fdp_status fdp_enqueue_pass(fdp_ctx *c, const fdp::DevTables &t, int L, const uint32_t *mods, uint32_t *main,
-                            uint32_t *blk, unsigned long long *acc, uint32_t *d_res, uint32_t *h_res,
+                            uint32_t *blk, uint32_t *esc, unsigned long long *acc, uint32_t *d_res, uint32_t *h_res,
                             unsigned int *d_err, cudaStream_t s, uint64_t *launches,
                             cudaStream_t span_stream = nullptr, cudaEvent_t fork = nullptr,
                             cudaEvent_t join = nullptr);

@@ -29,6 +29,7 @@
 #include "fdp_api_internal.h"
 #include "fdp_host.h"
 #include "fdp_launch.h"
+#include "fdp_tail_dev.h"
 
 namespace {
 
@@ -102,13 +103,17 @@ struct Job {
 
 // Bytes of one request in the pool: the state for `lanes` residues, then the
 // dot-product accumulators (256 bytes), and the device residues with the
-// request's error word 128 bytes after them (256 bytes).
-uint64_t request_bytes(int n, int lanes) {
+// request's error word 128 bytes after them (256 bytes); then, unless the
+// request would not fit the pool with them, the fused row tail's escape words.
+uint64_t request_bytes(int n, int lanes, uint64_t pool, bool *escapes = nullptr) {
   const int W = n + 1;
   const uint64_t M = fdp::main_states(W), D = fdp::blocked_states(W);
   const uint64_t a = (4ull * M * lanes + kAlign - 1) / kAlign * kAlign;
   const uint64_t b = (4ull * D * lanes + kAlign - 1) / kAlign * kAlign;
-  return a + b + 2 * kAlign;
+  const uint64_t e = (4ull * fdp::tail_escape_words(W) * lanes + kAlign - 1) / kAlign * kAlign;
+  const bool with = e > 0 && a + b + 2 * kAlign + e <= pool;
+  if (escapes) *escapes = with;
+  return a + b + 2 * kAlign + (with ? e : 0);
 }
 
 }  // namespace
@@ -151,7 +156,11 @@ struct fdp_server {
     char *base = pool + j->off;
     uint32_t *main = reinterpret_cast<uint32_t *>(base);
     uint32_t *blk = reinterpret_cast<uint32_t *>(base + (4ull * M * j->lanes + kAlign - 1) / kAlign * kAlign);
-    char *small = base + j->bytes - 2 * kAlign;
+    const uint64_t D = fdp::blocked_states(W);
+    char *small = reinterpret_cast<char *>(blk) + (4ull * D * j->lanes + kAlign - 1) / kAlign * kAlign;
+    bool escapes = false;
+    request_bytes(j->n, j->lanes, alloc.size, &escapes);
+    uint32_t *esc = escapes ? reinterpret_cast<uint32_t *>(small + 2 * kAlign) : nullptr;
     unsigned long long *acc = reinterpret_cast<unsigned long long *>(small);
     uint32_t *dres = reinterpret_cast<uint32_t *>(small + kAlign);
     unsigned int *derr = reinterpret_cast<unsigned int *>(small + kAlign + 128);
@@ -164,7 +173,7 @@ struct fdp_server {
     const std::vector<uint32_t> &mods = j->batch.empty() ? j->mods : j->batch;
     for (int done = 0; done < int(mods.size()) && es == FDP_OK; done += j->lanes) {
       const int L = std::min(j->lanes, int(mods.size()) - done);
-      es = fdp_enqueue_pass(ctx, *t, L, mods.data() + done, main, blk, acc, dres, pinned[size_t(slot)] + done,
+      es = fdp_enqueue_pass(ctx, *t, L, mods.data() + done, main, blk, esc, acc, dres, pinned[size_t(slot)] + done,
                             derr, s, &launches);
     }
     if (es == FDP_OK) es = fdp_cuda_status(fdp_enqueue_err_read(herr, derr, s), "serve: error word");
@@ -258,7 +267,7 @@ struct fdp_server {
               }
             }
           uint64_t off = 0;
-          uint64_t bytes = riders.empty() ? q->bytes : request_bytes(q->n, total);
+          uint64_t bytes = riders.empty() ? q->bytes : request_bytes(q->n, total, alloc.size);
           bool got = alloc.alloc(bytes, &off);
           if (!got && !riders.empty()) {  // the batch does not fit: the request alone
             riders.clear();
@@ -436,7 +445,7 @@ extern "C" fdp_status fdp_submit(fdp_ctx *c, const fdp_problem *pr, uint64_t *id
   j->mods.assign(pr->moduli, pr->moduli + pr->k);
   j->lanes = std::min(sv->cfg.max_lanes, pr->k);
   j->passes = (pr->k + j->lanes - 1) / j->lanes;
-  j->bytes = request_bytes(pr->n, j->lanes);
+  j->bytes = request_bytes(pr->n, j->lanes, sv->alloc.size);
   if (j->bytes > sv->alloc.size) {
     fdp_set_last_error("submit: request needs more device memory than the whole HBM budget");
     return FDP_ERR_HBM;

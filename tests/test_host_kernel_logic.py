@@ -3,7 +3,8 @@
 the sm_100a cell and growth kernels run is built here with g++ and checked on
 every cell of small widths, in every visiting order the kernel may use.  The
 row-k initialiser's automaton and fill plan (fdp_rowinit.cpp) are checked the
-same way against the oracle's state after the first rows."""
+same way against the oracle's state after the first rows, and the fused row
+tail's tables (fdp_tail.cpp) against the oracle's low cells."""
 import os
 import shutil
 import subprocess
@@ -42,5 +43,23 @@ def test_row_automaton_and_fill_match_oracle(tmp_path):
                     os.path.join(CSRC, "fdp_rowinit.cpp"), os.path.join(CSRC, "fdp_host.cpp"), str(oracle_o),
                     "-o", str(exe), "-lpthread"], check=True)
     out = subprocess.run([str(exe), "10"], capture_output=True, text=True, timeout=600)
+    assert out.returncode == 0, out.stdout + out.stderr
+    assert out.stdout.strip().endswith("bad=0"), out.stdout
+
+
+@pytest.mark.skipif(shutil.which("g++") is None or shutil.which("gcc") is None, reason="needs gcc/g++")
+@pytest.mark.skipif(not os.path.exists(os.path.join(CUDA_INC, "cuda_runtime.h")), reason="needs CUDA headers")
+def test_row_tail_tables_match_oracle(tmp_path):
+    # Every bottom width s = 2..W of widths 2..12, block by block from the
+    # highest end height down, with the escape slots between them.
+    oracle_o = tmp_path / "fdp_oracle.o"
+    subprocess.run(["gcc", "-O2", "-c", os.path.join(ROOT, "oracle", "fdp_oracle.c"), "-o", str(oracle_o)],
+                   check=True)
+    exe = tmp_path / "tail_check"
+    subprocess.run(["g++", "-O2", "-std=c++17", f"-I{CSRC}", f"-I{CUDA_INC}",
+                    os.path.join(ROOT, "tests", "host", "tail_check.cpp"),
+                    os.path.join(CSRC, "fdp_tail.cpp"), os.path.join(CSRC, "fdp_host.cpp"), str(oracle_o),
+                    "-o", str(exe), "-lpthread"], check=True)
+    out = subprocess.run([str(exe), "12"], capture_output=True, text=True, timeout=600)
     assert out.returncode == 0, out.stdout + out.stderr
     assert out.stdout.strip().endswith("bad=0"), out.stdout
