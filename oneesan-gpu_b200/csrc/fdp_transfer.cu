@@ -295,14 +295,25 @@ struct ApplyArgs {
   ull M, D;
   int K;
   uint32_t mod[16];
+  ull inv[16];  // floor((2^64 - 1) / mod)
 };
+
+// x mod p with m = floor((2^64 - 1) / p): the estimate of the quotient is at
+// most two short.
+__device__ __forceinline__ uint32_t reduce(ull x, uint32_t p, ull m) {
+  ull r = x - __umul64hi(x, m) * p;
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+    if (r >= p) r -= p;
+  return uint32_t(r);
+}
 
 __device__ __forceinline__ uint32_t src_value(const ApplyArgs &a, ull j, int l) {
   return j < a.M ? a.in_main[lane_addr(a.K, a.M, j, l)] : a.in_blk[lane_addr(a.K, a.D, j - a.M, l)];
 }
 
 __device__ __forceinline__ void store_row(const ApplyArgs &a, ull i, int l, ull sum) {
-  const uint32_t v = uint32_t(sum % a.mod[l]);  // sum < 2^41: at most ~6W sources below 2^32
+  const uint32_t v = reduce(sum, a.mod[l], a.inv[l]);  // sum < 2^41: at most ~6W sources below 2^32
   if (i < a.M) a.out_main[lane_addr(a.K, a.M, i, l)] = v;
   else a.out_blk[lane_addr(a.K, a.D, i - a.M, l)] = v;
 }
@@ -315,6 +326,67 @@ __global__ void csr_apply_kernel(ApplyArgs a, const ull *offsets, const uint32_t
       ull sum = i < a.M ? a.in_main[lane_addr(a.K, a.M, i, l)] : 0ull;
       for (ull k = b; k < e; ++k) sum += src_value(a, columns[k], l);
       store_row(a, i, l, sum);
+    }
+  }
+}
+
+// The same rows for K lanes at once: one read of the row's offsets and columns
+// serves every lane, and a source is one access per panel.  Needs the panels'
+// alignment; csr_apply_kernel takes other pointers.
+// Bound: HBM and the scattered source reads.  Width 16, 4 lanes, paired cells:
+// 113 -> 36 us (the lane loop around one row's walk read the row K times and
+// divided by the modulus at each output).
+template <int K>
+__global__ void __launch_bounds__(256) csr_apply_lanes_kernel(ApplyArgs a, const ull *offsets, const uint32_t *columns) {
+  const ull total = a.M + a.D;
+  for (ull i = ull(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += ull(gridDim.x) * blockDim.x) {
+    const ull b = offsets[i], e = offsets[i + 1];
+    ull sum[K];
+    uint32_t x[K];
+    if (i < a.M) fdp::ld_lanes<K>(a.in_main, a.M, i, x);
+#pragma unroll
+    for (int l = 0; l < K; ++l) sum[l] = i < a.M ? x[l] : 0u;
+    for (ull k = b; k < e; ++k) {
+      const ull j = columns[k];
+      if (j < a.M) fdp::ld_lanes<K>(a.in_main, a.M, j, x);
+      else fdp::ld_lanes<K>(a.in_blk, a.D, j - a.M, x);
+#pragma unroll
+      for (int l = 0; l < K; ++l) sum[l] += x[l];
+    }
+#pragma unroll
+    for (int l = 0; l < K; ++l) x[l] = reduce(sum[l], a.mod[l], a.inv[l]);
+    if (i < a.M) fdp::st_lanes<K>(a.out_main, a.M, i, x);
+    else fdp::st_lanes<K>(a.out_blk, a.D, i - a.M, x);
+  }
+}
+
+// Both input vectors to the outputs, each value reduced by its lane's modulus;
+// blockIdx.y is the panel.
+__global__ void __launch_bounds__(256) copy_residues_kernel(ApplyArgs a) {
+  int l0 = 0, pw = 0;
+  for (unsigned k = 0; k <= blockIdx.y; ++k) {
+    l0 += pw;
+    pw = (a.K - l0 >= 8) ? 8 : (a.K - l0 >= 4) ? 4 : (a.K - l0 >= 2) ? 2 : 1;
+  }
+  const ull nm = a.M * ull(pw), n = nm + a.D * ull(pw);
+  const uint32_t *im = a.in_main + ull(l0) * a.M, *ib = a.in_blk + ull(l0) * a.D;
+  uint32_t *om = a.out_main + ull(l0) * a.M, *ob = a.out_blk + ull(l0) * a.D;
+  auto one = [&](uint32_t v, int l) {
+    const uint32_t p = a.mod[l0 + l];
+    return v < p ? v : v % p;
+  };
+  if (pw >= 4) {
+    for (ull u = (ull(blockIdx.x) * blockDim.x + threadIdx.x) * 4; u < n; u += ull(gridDim.x) * blockDim.x * 4) {
+      const int l = int(u & ull(pw - 1));
+      uint4 v = *reinterpret_cast<const uint4 *>(u < nm ? im + u : ib + (u - nm));
+      v = make_uint4(one(v.x, l), one(v.y, l + 1), one(v.z, l + 2), one(v.w, l + 3));
+      *reinterpret_cast<uint4 *>(u < nm ? om + u : ob + (u - nm)) = v;
+    }
+  } else {
+    for (ull u = ull(blockIdx.x) * blockDim.x + threadIdx.x; u < n; u += ull(gridDim.x) * blockDim.x) {
+      const int l = int(u & ull(pw - 1));
+      if (u < nm) om[u] = one(im[u], l);
+      else ob[u - nm] = one(ib[u - nm], l);
     }
   }
 }
@@ -375,6 +447,9 @@ fdp_status check_apply(int width, int lanes, const uint32_t *moduli, const void 
 }
 
 }  // namespace
+
+// Main and blocked words from which reverse2 runs as two in-place cells.
+static constexpr ull kReverse2InPlace = 512;
 
 struct fdp_transfer_map {
   int device = 0, width = 0, p = 0, paired = 0;
@@ -497,7 +572,10 @@ static fdp_status launch_apply(fdp_ctx *c, int width, int lanes, const uint32_t 
   a->M = fdp::main_states(width);
   a->D = fdp::blocked_states(width);
   a->K = lanes;
-  for (int i = 0; i < lanes; ++i) a->mod[i] = moduli[i];
+  for (int i = 0; i < lanes; ++i) {
+    a->mod[i] = moduli[i];
+    a->inv[i] = ~0ull / moduli[i];
+  }
   (void)c;
   (void)stream;
   return FDP_OK;
@@ -514,7 +592,20 @@ extern "C" fdp_status fdp_transfer_map_apply(fdp_ctx *c, const fdp_transfer_map 
   ApplyArgs a{};
   launch_apply(c, m->width, lanes, moduli, d_in_main, d_in_block, d_out_main, d_out_block, stream, &a);
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : c->stream;
-  csr_apply_kernel<<<grid_for(m->rows), 256, 0, st>>>(a, m->offsets, m->columns);
+  const bool aligned = fdp::panel_aligned(lanes, d_in_main) && fdp::panel_aligned(lanes, d_in_block) &&
+                       fdp::panel_aligned(lanes, d_out_main) && fdp::panel_aligned(lanes, d_out_block);
+  if (!aligned) {
+    csr_apply_kernel<<<grid_for(m->rows), 256, 0, st>>>(a, m->offsets, m->columns);
+    return fdp_cuda_status(cudaGetLastError(), "csr apply");
+  }
+  const unsigned blocks = unsigned((m->rows + 255) / 256);
+#define APPLY_K(k) \
+  case k: csr_apply_lanes_kernel<k><<<blocks, 256, 0, st>>>(a, m->offsets, m->columns); break;
+  switch (lanes) {
+    APPLY_K(1) APPLY_K(2) APPLY_K(3) APPLY_K(4) APPLY_K(5) APPLY_K(6) APPLY_K(7) APPLY_K(8)
+    APPLY_K(9) APPLY_K(10) APPLY_K(11) APPLY_K(12) APPLY_K(13) APPLY_K(14) APPLY_K(15) APPLY_K(16)
+  }
+#undef APPLY_K
   return fdp_cuda_status(cudaGetLastError(), "csr apply");
 }
 
@@ -534,6 +625,26 @@ extern "C" fdp_status fdp_reverse2_apply(fdp_ctx *c, int width, int p, int lanes
   ApplyArgs a{};
   launch_apply(c, width, lanes, moduli, d_in_main, d_in_block, d_out_main, d_out_block, stream, &a);
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : c->stream;
+  // The inputs, reduced, go to the outputs, and the two cells run there in place:
+  // no ranks of sources, whole panel words.  Unaligned pointers, tiny vectors and
+  // streams under capture (the width's tables may have to be uploaded) enumerate
+  // the sources of the sources.  The line: three launches take 20 us, the
+  // enumeration 23 us for one lane of width 8 (708 words), 816 against 41 us for
+  // 8 lanes of width 15.
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  const bool aligned = fdp::panel_aligned(lanes, d_in_main) && fdp::panel_aligned(lanes, d_in_block) &&
+                       fdp::panel_aligned(lanes, d_out_main) && fdp::panel_aligned(lanes, d_out_block);
+  if (aligned && (a.M + a.D) * ull(lanes) >= kReverse2InPlace &&
+      cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
+    const fdp::DevTables *t = nullptr;
+    if ((s = fdp_ctx_tables(c, width, &t)) != FDP_OK) return s;
+    const int panels = lanes / 8 + __builtin_popcount(unsigned(lanes % 8));
+    copy_residues_kernel<<<dim3(grid_for(a.M + a.D), unsigned(panels)), 256, 0, st>>>(a);
+    e = cudaGetLastError();
+    for (int q = p; q >= p - 1 && e == cudaSuccess; --q)
+      e = fdp::launch_cell(*t, lanes, moduli, d_out_main, d_out_block, q, false, true, fdp::LaunchCfg{}, st);
+    return fdp_cuda_status(e, "reverse2");
+  }
   reverse2_kernel<<<grid_for(a.M + a.D), 256, 0, st>>>(a, cnt, width, p);
   return fdp_cuda_status(cudaGetLastError(), "reverse2");
 }
@@ -597,52 +708,95 @@ struct GroupArgs {
   int W, fixed;
   uint32_t occ0;
   ull gm, total;  // group main rows, main + blocked rows
-  int G;
-  const uint32_t *masks;
+  uint32_t masks[32];
 };
 
-__global__ void group_gather_kernel(GroupArgs a, const uint32_t *in_main, const uint32_t *in_blk, uint32_t *arena,
-                                    ull *ranks) {
-  __shared__ ull sG[FDP_MAXW + 1][FDP_HT];
-  __shared__ ull sF[FDP_MAXW + 1][FDP_HT];
-  for (int k = threadIdx.x; k < (FDP_MAXW + 1) * FDP_HT; k += blockDim.x) {
-    (&sG[0][0])[k] = (&a.gcounts->H[0][0])[k];
-    (&sF[0][0])[k] = (&a.full->H[0][0])[k];
-  }
+// Counts of words of up to W symbols in the rank type, in shared memory.
+template <typename Idx>
+__device__ __forceinline__ void load_counts_as(Idx (*s)[FDP_HT], const Counts *c, int W) {
+  for (int k = threadIdx.x; k < W * FDP_HT; k += blockDim.x) (&s[0][0])[k] = Idx((&c->H[0][0])[k]);
+}
+
+// Local row i of group blockIdx.y (word and global rank) at arena[g * total +
+// i]: neighbouring threads take neighbouring rows of one group, whose global
+// ranks lie close together.  The local word is unranked, moved to the group's
+// positions and ranked in one walk each, in 32 bits where the width's ranks fit.
+template <typename Idx>
+__global__ void __launch_bounds__(256) group_gather_kernel(const __grid_constant__ GroupArgs a, const uint32_t *in_main,
+                                                           const uint32_t *in_blk, uint32_t *arena, ull *ranks) {
+  __shared__ Idx sG[FDP_MAXW][FDP_HT], sF[FDP_MAXW][FDP_HT];
+  load_counts_as<Idx>(sG, a.gcounts, a.W);
+  load_counts_as<Idx>(sF, a.full, a.W);
   __syncthreads();
-  const GroupSpace gs{sG, a.fixed, a.occ0};
-  const ull n = a.total * ull(a.G);
-  for (ull idx = ull(blockIdx.x) * blockDim.x + threadIdx.x; idx < n; idx += ull(gridDim.x) * blockDim.x) {
-    const ull i = idx / ull(a.G);
-    const int g = int(idx - i * ull(a.G));
+  const uint32_t mask = a.masks[blockIdx.y];
+  const ull row0 = ull(blockIdx.y) * a.total;
+  for (ull i = ull(blockIdx.x) * blockDim.x + threadIdx.x; i < a.total; i += ull(gridDim.x) * blockDim.x) {
     const bool is_main = i < a.gm;
     const int width = is_main ? a.W : a.W - 1;
-    const uint64_t w = move_occupied(gs.unrank(is_main ? i : i - a.gm, width), a.occ0, a.masks[g], a.fixed);
-    const ull r = rank_word_dev(w, width, sF);
-    ranks[idx] = r;
-    arena[idx] = is_main ? in_main[r] : in_blk[r];
+    Idx r = Idx(is_main ? i : i - a.gm);
+    uint64_t w = 0;
+    int h = 1;
+    for (int pos = width - 1; pos >= 0; --pos) {
+      const bool held = pos < a.fixed, occ = (a.occ0 >> pos) & 1u;
+      const Idx zN = held && occ ? Idx(0) : sG[pos][h], below = sG[pos][h > 0 ? h - 1 : 0];
+      const Idx zR = zN + (h > 0 && !(held && !occ) ? below : Idx(0));
+      const bool ge1 = r >= zN, ge2 = r >= zR;
+      r -= ge2 ? zR : (ge1 ? zN : Idx(0));
+      w = (w << 2) | (ge2 ? fdp::SYM_L : (ge1 ? fdp::SYM_R : fdp::SYM_N));
+      h += ge2 ? 1 : (ge1 ? -1 : 0);
+    }
+    w = move_occupied(w, a.occ0, mask, a.fixed);
+    Idx g = 0;
+    h = 1;
+    for (int pos = width - 1; pos >= 0; --pos) {
+      const uint32_t s = get(w, pos);
+      if (s != fdp::SYM_N) g += sF[pos][h];
+      if (s == fdp::SYM_L && h > 0) g += sF[pos][h - 1];
+      h += s == fdp::SYM_L ? 1 : (s == fdp::SYM_R ? -1 : 0);
+    }
+    ranks[row0 + i] = ull(g);
+    arena[row0 + i] = is_main ? in_main[g] : in_blk[g];
   }
 }
 
-__global__ void group_apply_kernel(GroupArgs a, const uint32_t *arena_in, uint32_t *arena_out, const ull *offsets,
-                                   const uint32_t *columns, uint32_t mod) {
-  const ull n = a.total * ull(a.G);
-  for (ull idx = ull(blockIdx.x) * blockDim.x + threadIdx.x; idx < n; idx += ull(gridDim.x) * blockDim.x) {
-    const ull i = idx / ull(a.G);
-    const ull g = idx - i * ull(a.G);
-    ull sum = i < a.gm ? arena_in[idx] : 0ull;
-    for (ull e = offsets[i]; e < offsets[i + 1]; ++e) sum += arena_in[ull(columns[e]) * ull(a.G) + g];
-    arena_out[idx] = uint32_t(sum % mod);  // sum < 2^41: at most ~6W sources below 2^32
-  }
+// One row of one group: its sources' sum mod p.
+__device__ __forceinline__ uint32_t group_row(const GroupArgs &a, const uint32_t *arena, const ull *offsets,
+                                              const uint32_t *columns, uint32_t mod, ull inv, ull i) {
+  ull sum = i < a.gm ? arena[i] : 0ull;
+  for (ull e = offsets[i], end = offsets[i + 1]; e < end; ++e) sum += arena[columns[e]];
+  return reduce(sum, mod, inv);  // sum < 2^41: at most ~6W sources below 2^32
 }
 
-__global__ void group_scatter_kernel(GroupArgs a, const uint32_t *arena_out, const ull *ranks, uint32_t *out_main,
-                                     uint32_t *out_blk) {
-  const ull n = a.total * ull(a.G);
-  for (ull idx = ull(blockIdx.x) * blockDim.x + threadIdx.x; idx < n; idx += ull(gridDim.x) * blockDim.x) {
-    const ull i = idx / ull(a.G);
-    (i < a.gm ? out_main : out_blk)[ranks[idx]] = arena_out[idx];
-  }
+// The apply written straight to the global ranks.  Bound: launches and latency
+// (a group holds 10^4 to 10^5 rows).  Width 17, 70 groups of 4 of 8
+// positions, three calls: 94 -> 81 us with this, the masks as kernel arguments
+// instead of a copy, and the rows of a group side by side.
+__global__ void __launch_bounds__(256) group_apply_scatter_kernel(const __grid_constant__ GroupArgs a,
+                                                                  const uint32_t *arena_in, const ull *ranks,
+                                                                  const ull *offsets, const uint32_t *columns,
+                                                                  uint32_t mod, ull inv, uint32_t *out_main,
+                                                                  uint32_t *out_blk) {
+  const ull row0 = ull(blockIdx.y) * a.total;
+  for (ull i = ull(blockIdx.x) * blockDim.x + threadIdx.x; i < a.total; i += ull(gridDim.x) * blockDim.x)
+    (i < a.gm ? out_main : out_blk)[ranks[row0 + i]] =
+        group_row(a, arena_in + row0, offsets, columns, mod, inv, i);
+}
+
+// The two halves apart, for the phase timers.
+__global__ void __launch_bounds__(256) group_apply_kernel(const __grid_constant__ GroupArgs a, const uint32_t *arena_in,
+                                                          uint32_t *arena_out, const ull *offsets,
+                                                          const uint32_t *columns, uint32_t mod, ull inv) {
+  const ull row0 = ull(blockIdx.y) * a.total;
+  for (ull i = ull(blockIdx.x) * blockDim.x + threadIdx.x; i < a.total; i += ull(gridDim.x) * blockDim.x)
+    arena_out[row0 + i] = group_row(a, arena_in + row0, offsets, columns, mod, inv, i);
+}
+
+__global__ void __launch_bounds__(256) group_scatter_kernel(const __grid_constant__ GroupArgs a,
+                                                            const uint32_t *arena_out, const ull *ranks,
+                                                            uint32_t *out_main, uint32_t *out_blk) {
+  const ull row0 = ull(blockIdx.y) * a.total;
+  for (ull i = ull(blockIdx.x) * blockDim.x + threadIdx.x; i < a.total; i += ull(gridDim.x) * blockDim.x)
+    (i < a.gm ? out_main : out_blk)[ranks[row0 + i]] = arena_out[row0 + i];
 }
 
 }  // namespace
@@ -653,12 +807,12 @@ struct fdp_factor_map {
   ull *offsets = nullptr;
   uint32_t *columns = nullptr;
   Counts *gcounts = nullptr;
-  uint32_t *masks = nullptr, *arena_in = nullptr, *arena_out = nullptr;
+  uint32_t *arena_in = nullptr, *arena_out = nullptr;
   ull *ranks = nullptr;
   cudaEvent_t ev[4] = {};
   ~fdp_factor_map() {
     cudaSetDevice(device);
-    for (void *q : {(void *)offsets, (void *)columns, (void *)gcounts, (void *)masks, (void *)arena_in,
+    for (void *q : {(void *)offsets, (void *)columns, (void *)gcounts, (void *)arena_in,
                     (void *)arena_out, (void *)ranks})
       if (q) cudaFree(q);
     for (cudaEvent_t e : ev)
@@ -703,7 +857,6 @@ extern "C" fdp_status fdp_factor_map_build(fdp_ctx *c, int width, int p, int pai
   const size_t cells = size_t(total) * size_t(max_groups);
   if ((e = cudaMalloc(&map->gcounts, sizeof(Counts))) != cudaSuccess ||
       (e = cudaMemcpy(map->gcounts, &hg, sizeof(Counts), cudaMemcpyHostToDevice)) != cudaSuccess ||
-      (e = cudaMalloc(&map->masks, sizeof(uint32_t) * 32)) != cudaSuccess ||
       (e = cudaMalloc(&map->arena_in, sizeof(uint32_t) * cells)) != cudaSuccess ||
       (e = cudaMalloc(&map->arena_out, sizeof(uint32_t) * cells)) != cudaSuccess ||
       (e = cudaMalloc(&map->ranks, sizeof(ull) * cells)) != cudaSuccess)
@@ -725,7 +878,7 @@ extern "C" fdp_status fdp_factor_map_info(const fdp_factor_map *m, uint64_t *gro
   if (group_blocked) *group_blocked = m->gd;
   if (edges) *edges = m->edges;
   if (device_bytes)
-    *device_bytes = sizeof(ull) * (rows + 1) + sizeof(uint32_t) * m->edges + sizeof(Counts) + 4 * 32 +
+    *device_bytes = sizeof(ull) * (rows + 1) + sizeof(uint32_t) * m->edges + sizeof(Counts) +
                     cells * (2 * sizeof(uint32_t) + sizeof(ull));
   return FDP_OK;
 }
@@ -750,27 +903,30 @@ extern "C" fdp_status fdp_factor_map_apply(fdp_ctx *c, const fdp_factor_map *m, 
   const Counts *full = device_counts();
   if (!full) return FDP_ERR_HBM;
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : c->stream;
-  if ((e = cudaMemcpyAsync(m->masks, masks, sizeof(uint32_t) * size_t(groups), cudaMemcpyHostToDevice, st)) !=
-      cudaSuccess)
-    return fdp_cuda_status(e, "factor map masks");
   GroupArgs a{m->gcounts, full, m->width, m->fixed, m->occupied ? (1u << m->occupied) - 1u : 0u,
-              m->gm, m->gm + m->gd, groups, m->masks};
-  const unsigned grid = grid_for(a.total * ull(groups));
+              m->gm, m->gm + m->gd, {}};
+  for (int g = 0; g < groups; ++g) a.masks[g] = masks[g];
+  const ull inv = ~0ull / modulus;
+  const dim3 grid(grid_for(a.total), unsigned(groups));
   if (phase_ms) cudaEventRecord(m->ev[0], st);
-  group_gather_kernel<<<grid, 256, 0, st>>>(a, d_in_main, d_in_block, m->arena_in, m->ranks);
-  if (phase_ms) cudaEventRecord(m->ev[1], st);
-  group_apply_kernel<<<grid, 256, 0, st>>>(a, m->arena_in, m->arena_out, m->offsets, m->columns, modulus);
-  if (phase_ms) cudaEventRecord(m->ev[2], st);
+  if (fdp::needs_u64(m->width)) group_gather_kernel<ull><<<grid, 256, 0, st>>>(a, d_in_main, d_in_block, m->arena_in, m->ranks);
+  else group_gather_kernel<uint32_t><<<grid, 256, 0, st>>>(a, d_in_main, d_in_block, m->arena_in, m->ranks);
+  if (!phase_ms) {
+    group_apply_scatter_kernel<<<grid, 256, 0, st>>>(a, m->arena_in, m->ranks, m->offsets, m->columns, modulus, inv,
+                                                     d_out_main, d_out_block);
+    return fdp_cuda_status(cudaGetLastError(), "factor map apply");
+  }
+  cudaEventRecord(m->ev[1], st);
+  group_apply_kernel<<<grid, 256, 0, st>>>(a, m->arena_in, m->arena_out, m->offsets, m->columns, modulus, inv);
+  cudaEventRecord(m->ev[2], st);
   group_scatter_kernel<<<grid, 256, 0, st>>>(a, m->arena_out, m->ranks, d_out_main, d_out_block);
-  if (phase_ms) cudaEventRecord(m->ev[3], st);
+  cudaEventRecord(m->ev[3], st);
   if ((e = cudaGetLastError()) != cudaSuccess) return fdp_cuda_status(e, "factor map apply");
-  if (phase_ms) {
-    if ((e = cudaEventSynchronize(m->ev[3])) != cudaSuccess) return fdp_cuda_status(e, "factor map apply");
-    for (int k = 0; k < 3; ++k) {
-      float ms = 0;
-      cudaEventElapsedTime(&ms, m->ev[k], m->ev[k + 1]);
-      phase_ms[k] = ms;
-    }
+  if ((e = cudaEventSynchronize(m->ev[3])) != cudaSuccess) return fdp_cuda_status(e, "factor map apply");
+  for (int k = 0; k < 3; ++k) {
+    float ms = 0;
+    cudaEventElapsedTime(&ms, m->ev[k], m->ev[k + 1]);
+    phase_ms[k] = ms;
   }
   return FDP_OK;
 }
