@@ -215,6 +215,12 @@ static int row_init_rows(const fdp_ctx *c, int W, int *cap) {
   return fit_row_init(W, R, c->cfg.bounded_prefix, cap);
 }
 
+// Whether a pass of width W is one launch with the state in shared memory: small
+// widths, unless the tuning asks for a particular way through the first rows.
+static bool whole_pass(const fdp_ctx *c, int W) {
+  return c->cfg.tail && fdp::solves_whole(W) && c->cfg.row_init == 0 && c->cfg.bounded_prefix;
+}
+
 // Every device table a residue pass of width W reads, uploaded before any
 // stream capture starts (allocation and blocking copies cannot be captured).
 fdp_status fdp_prepare_pass(fdp_ctx *c, int W, const DevTables **full) {
@@ -222,6 +228,10 @@ fdp_status fdp_prepare_pass(fdp_ctx *c, int W, const DevTables **full) {
   if (s != FDP_OK) return s;
   int rcap = 0;
   if (const int R = row_init_rows(c, W, &rcap)) FDP_CK(fdp::prepare_row_init(W, R, rcap), "row-k initialiser tables");
+  if (whole_pass(c, W)) {
+    FDP_CK(fdp::prepare_whole(W), "whole-solve tables");
+    return FDP_OK;
+  }
   if (c->cfg.tail) FDP_CK(fdp::prepare_tail(W), "row tail tables");
   if (!c->cfg.bounded_prefix || W < 4) return s;
   std::vector<int> caps = fdp::bounded_prefix_caps(W);
@@ -301,6 +311,12 @@ fdp_status fdp_enqueue_pass(fdp_ctx *c, const DevTables &t, int L, const uint32_
                             unsigned int *d_err, cudaStream_t s, uint64_t *launches, cudaStream_t span_stream,
                             cudaEvent_t fork, cudaEvent_t join) {
   const int W = t.W;
+  if (whole_pass(c, W)) {
+    FDP_CK(fdp::launch_whole(W, L, mods, d_res, s), "whole solve");
+    if (h_res) FDP_CK(cudaMemcpyAsync(h_res, d_res, sizeof(uint32_t) * L, cudaMemcpyDeviceToHost, s), "residue copy");
+    if (launches) ++*launches;
+    return FDP_OK;
+  }
   const uint64_t M = fdp::main_states(W), D = fdp::blocked_states(W);
   uint64_t n = 0;
   fdp_status st = FDP_OK;

@@ -88,7 +88,7 @@ std::vector<uint32_t> tail_words(int s, int g) {
   return w;  // built in lexicographic, so numeric, order
 }
 
-TailTables build_tail_tables(int s) {
+static TailTables build_tables(int s, bool whole) {
   TailTables t;
   t.s = s;
   t.cls.resize(size_t(s) + 1);
@@ -101,11 +101,12 @@ TailTables build_tail_tables(int s) {
   // stays at or above the height h' >= 2 above the pair.
   std::vector<std::vector<std::vector<uint32_t>>> esc(size_t(s) + 1, std::vector<std::vector<uint32_t>>(size_t(s)));
   for (int g = 0; g <= s; ++g) {
+    if (whole && g != 1) continue;
     TailClass &c = t.cls[size_t(g)];
     c = TailClass{};
     c.nmain = uint32_t(mw[size_t(g)].size());
     c.nblk = uint32_t(bw[size_t(g)].size());
-    for (int p = s - 1; p >= 1; --p) {
+    for (int p = s - 1; p >= 1 && !whole; --p) {
       auto &e = esc[size_t(g)][size_t(p)];
       TailCell &cell = c.cell[p];
       cell.o0 = uint32_t(t.out.size());
@@ -123,6 +124,7 @@ TailTables build_tail_tables(int s) {
     }
   }
   for (int g = 0; g <= s; ++g) {
+    if (whole && g != 1) continue;
     TailClass &c = t.cls[size_t(g)];
     const auto &W = mw[size_t(g)], &B = bw[size_t(g)];
     const uint32_t zero = c.nmain;
@@ -189,7 +191,7 @@ TailTables build_tail_tables(int s) {
       cell.nn = uint32_t(items.size());
       cell.nx = uint32_t(xs.size());
       items.insert(items.end(), xs.begin(), xs.end());
-      for (size_t i = 0, e; i < items.size(); i = e) {
+      for (size_t i = 0, e; i < items.size() && !whole; i = e) {
         for (e = i + 1; e < items.size() && items[e].src.size() == items[i].src.size() && (e < cell.nn) == (i < cell.nn);) ++e;
         spread_banks(items, i, e);
       }
@@ -212,6 +214,9 @@ TailTables build_tail_tables(int s) {
   }
   return t;
 }
+
+TailTables build_tail_tables(int s) { return build_tables(s, false); }
+TailTables build_whole_tables(int W) { return build_tables(W, true); }
 
 const TopCounts &top_counts(int g) {
   static const std::vector<TopCounts> all = [] {

@@ -58,7 +58,7 @@ struct TailClass {
 };
 
 struct TailTables {
-  int s = 0;
+  int s = 0;  // (build_whole_tables fills cls[1] alone)
   std::vector<TailClass> cls;  // by g, 0..s
   std::vector<uint32_t> item;  // four words each
   std::vector<uint32_t> more;  // two words for each item
@@ -68,6 +68,10 @@ struct TailTables {
 
 // Tables for bottom parts of s symbols, every end height 0..s (2 <= s <= 12).
 TailTables build_tail_tables(int s);
+
+// The whole space of a width W <= 12 as one block (end height 1, no top part and
+// so no escapes), items in canonical order within like numbers of sources.
+TailTables build_whole_tables(int W);
 
 // Local code of bottom word `i` of class g: two bits a symbol, canonical order.
 std::vector<uint32_t> tail_words(int s, int g);

@@ -408,6 +408,105 @@ __global__ void __launch_bounds__(kThreads, 2) tail_kernel(const __grid_constant
   }
 }
 
+// One lane of a whole solve, its state in shared memory: the first-row state,
+// W - 2 rows of cells, the dot product with the first-row state.  One barrier a
+// cell, no launch between cells.
+// Bound: the latency of a cell (barrier, shared-memory round trips) up to n = 9,
+// the item tables' L2 reads (16 bytes an item and cell) at n = 11.  Launching
+// each cell costs 8 to 11 us: device time of a pass, n = 9, two lanes 688 -> 89 us,
+// n = 10 849 -> 174 us.
+struct WholeArgs {
+  const uint4 *item;
+  const uint2 *more;
+  const uint16_t *first;  // local words of the 2^(W-1) first-row states
+  uint32_t *residues;
+  uint32_t mod[16];
+  int W;
+  TailClass cls;
+};
+
+constexpr int kWholeAhead = 4;
+
+__global__ void __launch_bounds__(1024, 1) whole_kernel(const __grid_constant__ WholeArgs a) {
+  extern __shared__ __align__(16) uint32_t w[];
+  __shared__ unsigned long long part[32];
+  const uint32_t tid = threadIdx.x, nthr = blockDim.x;
+  const uint32_t p_ = a.mod[blockIdx.x], nfirst = 1u << (a.W - 1);
+  const TailClass &c = a.cls;
+  for (uint32_t i = tid; i < c.words; i += nthr) w[i] = 0;
+  __syncthreads();
+  for (uint32_t i = tid; i < nfirst; i += nthr) w[a.first[i]] = 1u;
+  uint4 ahead[kWholeAhead];
+  auto read_ahead = [&](const TailCell &q) {
+    const uint32_t n = q.nn + q.nx;
+#pragma unroll
+    for (int k = 0; k < kWholeAhead; ++k) {
+      const uint32_t u = tid + uint32_t(k) * nthr;
+      if (u < n) ahead[k] = a.item[q.i0 + u];
+    }
+  };
+  auto item_n = [&](const uint4 &it, uint32_t i, bool last) {
+    const uint32_t nn = it.x & 0xffffu, lr = it.x >> 16, bl = it.y & 0xffffu, count = it.y >> 16;
+    uint32_t acc = count > 0 ? w[it.z & 0xffffu] : 0u;
+    if (count > 1) acc = add_mod(acc, w[it.z >> 16], p_);
+    if (count > 2) {
+      acc = add_mod(acc, w[it.w & 0xffffu], p_);
+      acc = add_mod(acc, w[it.w >> 16], p_);  // the zero word past the last source
+      if (count > 4) {
+        const uint2 e = a.more[i];
+        acc = add_mod(add_mod(acc, w[e.x & 0xffffu], p_), w[e.x >> 16], p_);
+        acc = add_mod(add_mod(acc, w[e.y & 0xffffu], p_), w[e.y >> 16], p_);
+      }
+    }
+    const uint32_t v = w[nn], vb = w[bl], vl = w[lr];
+    w[lr] = add_mod(vl, v, p_);
+    const uint32_t vn = add_mod(v, vb, p_);
+    w[nn] = last ? add_mod(vn, acc, p_) : vn;
+    w[bl] = last ? 0u : acc;
+  };
+  auto item_x = [&](const uint4 &it, bool last) {
+    const uint32_t own = it.x & 0xffffu, oth = it.x >> 16, bl = it.y;
+    const uint32_t vo = w[own], vx = w[oth], sum = add_mod(vo, vx, p_);
+    w[own] = add_mod(sum, w[bl], p_);
+    if (last) w[oth] = sum;
+    w[bl] = last ? 0u : vo;  // the next row starts without blocked words
+  };
+  const int rows = a.W >= 3 ? a.W - 2 : 0;
+  if (rows) read_ahead(c.cell[a.W - 1]);
+  for (int row = 0; row < rows; ++row)
+    for (int p = a.W - 1; p >= 1; --p) {
+      const TailCell &q = c.cell[p];
+      const uint32_t n = q.nn + q.nx;
+      uint4 now[kWholeAhead];
+#pragma unroll
+      for (int k = 0; k < kWholeAhead; ++k) now[k] = ahead[k];
+      read_ahead(c.cell[p > 1 ? p - 1 : a.W - 1]);
+      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < kWholeAhead; ++k) {
+        const uint32_t u = tid + uint32_t(k) * nthr;
+        if (u < q.nn) item_n(now[k], q.i0 + u, p == 1);
+        else if (u < n) item_x(now[k], p == 1);
+      }
+#pragma unroll 4
+      for (uint32_t u = tid + kWholeAhead * nthr; u < n; u += nthr) {
+        const uint4 it = a.item[q.i0 + u];
+        if (u < q.nn) item_n(it, q.i0 + u, p == 1);
+        else item_x(it, p == 1);
+      }
+    }
+  __syncthreads();
+  unsigned long long acc = 0;
+  for (uint32_t i = tid; i < nfirst; i += nthr) acc += w[a.first[i]];
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+  if ((tid & 31) == 0) part[tid >> 5] = acc;
+  __syncthreads();
+  if (tid == 0) {
+    for (uint32_t k = 1; k < nthr / 32; ++k) acc += part[k];
+    a.residues[blockIdx.x] = uint32_t(acc % p_);
+  }
+}
+
 template <typename Idx>
 constexpr size_t blocks_bytes() { return (sizeof(TailBlocks<Idx>) + 31) & ~size_t(31); }
 
@@ -471,6 +570,62 @@ cudaError_t tail_device(int s, TailDevice **out) {
 }
 
 }  // namespace
+
+struct WholeDevice {
+  TailClass cls;
+  uint4 *item = nullptr;
+  uint2 *more = nullptr;
+  uint16_t *first = nullptr;
+};
+
+static std::map<std::pair<int, int>, WholeDevice> g_whole;  // (device, W), guarded by g_mu
+
+bool solves_whole(int W) { return W <= 12; }
+
+cudaError_t prepare_whole(int W) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lk(g_mu);
+  if (g_whole.count({dev, W})) return cudaSuccess;
+  static std::map<std::pair<int, int>, std::unique_ptr<TailDevice>> owners;  // free the arrays at exit
+  const TailTables t = build_whole_tables(W);
+  auto d = std::make_unique<TailDevice>();
+  WholeDevice wd;
+  wd.cls = t.cls[1];
+  std::vector<uint16_t> first;
+  for (uint64_t m = 0; m < (1ull << (W - 1)); ++m) first.push_back(uint16_t(rank_word(first_row_state(m, W), W)));
+  if ((e = upload(*d, t.item, &wd.item)) != cudaSuccess) return e;
+  if ((e = upload(*d, t.more, &wd.more)) != cudaSuccess) return e;
+  if ((e = upload(*d, first, &wd.first)) != cudaSuccess) return e;
+  if ((e = cudaFuncSetAttribute(whole_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)) != cudaSuccess)
+    return e;
+  owners[{dev, W}] = std::move(d);
+  g_whole[{dev, W}] = wd;
+  return cudaSuccess;
+}
+
+cudaError_t launch_whole(int W, int K, const uint32_t *mods, uint32_t *residues, cudaStream_t st) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  WholeArgs a{};
+  {
+    std::lock_guard<std::mutex> lk(g_mu);
+    auto it = g_whole.find({dev, W});
+    if (it == g_whole.end()) return cudaErrorNotReady;  // prepare_whole first (outside capture)
+    a.item = it->second.item;
+    a.more = it->second.more;
+    a.first = it->second.first;
+    a.cls = it->second.cls;
+  }
+  a.residues = residues;
+  a.W = W;
+  for (int l = 0; l < K; ++l) a.mod[l] = mods[l];
+  const unsigned threads = std::min(1024u, std::max(64u, (a.cls.nblk + 31) / 32 * 32));
+  whole_kernel<<<unsigned(K), threads, size_t(a.cls.words) * 4, st>>>(a);
+  return cudaGetLastError();
+}
 
 int tail_symbols(int W) { return W >= 14 ? 9 : 0; }
 

@@ -20,4 +20,10 @@ cudaError_t prepare_tail(int W);
 cudaError_t launch_tail(const DevTables &t, int K, const uint32_t *mods, uint32_t *main, const uint32_t *blk,
                         uint32_t *esc, cudaStream_t s, uint64_t *launches);
 
+// Small widths: the whole residue computation of K lanes in one launch, each
+// lane's state in the shared memory of one CTA; residues[l] is the result.
+bool solves_whole(int W);
+cudaError_t prepare_whole(int W);  // tables, once per device; outside stream capture
+cudaError_t launch_whole(int W, int K, const uint32_t *mods, uint32_t *residues, cudaStream_t s);
+
 }  // namespace fdp
