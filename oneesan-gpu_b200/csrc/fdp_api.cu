@@ -22,6 +22,8 @@ static thread_local std::string g_last_error;
 // Device memory left free beside an escape buffer.
 static constexpr size_t kEscapeMargin = size_t(1) << 30;
 static constexpr size_t kWindowEscapes = size_t(1) << 30;
+// Device memory fdp_run_multi_sync keeps for its next call.
+static constexpr size_t kMultiKeep = size_t(2) << 30;
 
 static fdp_status cuda_status(cudaError_t e, const char *what) {
   if (e == cudaSuccess) return FDP_OK;
@@ -159,6 +161,10 @@ fdp_ctx::~fdp_ctx() {
   if (d_main) cudaFree(d_main);
   if (d_blk) cudaFree(d_blk);
   if (d_esc) cudaFree(d_esc);
+  if (d_multi) cudaFree(d_multi);
+  if (h_multi) cudaFreeHost(h_multi);
+  for (cudaStream_t x : multi_streams) cudaStreamDestroy(x);
+  for (cudaEvent_t x : multi_events) cudaEventDestroy(x);
   if (d_acc) cudaFree(d_acc);
   if (d_res) cudaFree(d_res);
   if (h_res) cudaFreeHost(h_res);
@@ -265,6 +271,11 @@ static fdp_status ensure_state(fdp_ctx *c, int W, int lanes, bool want_esc) {
     cudaFree(c->d_esc);
     c->d_esc = nullptr;
     c->cap_esc = 0;
+  }
+  if (c->d_multi && (c->cap_main < mb || c->cap_blk < bb)) {
+    cudaFree(c->d_multi);
+    c->d_multi = nullptr;
+    c->cap_multi = 0;
   }
   fdp_status s = ensure_buffer(&c->d_main, &c->cap_main, mb, "main state");
   if (s == FDP_OK) s = ensure_buffer(&c->d_blk, &c->cap_blk, bb, "blocked state");
@@ -423,7 +434,7 @@ extern "C" fdp_status fdp_run_sync(fdp_ctx *c, const fdp_problem *pr, uint32_t *
   const DevTables *t = nullptr;
   if ((s = fdp_prepare_pass(c, W, &t)) != FDP_OK) return s;
   const int lanes = pr->lanes < pr->k ? pr->lanes : pr->k;
-  if ((s = ensure_state(c, W, lanes, c->cfg.tail)) != FDP_OK) return s;
+  if (!whole_pass(c, W) && (s = ensure_state(c, W, lanes, c->cfg.tail)) != FDP_OK) return s;
   // Every pass (lanes residues each) is captured into ONE graph, run with one launch.
   fdp_run_stats acc{};
   auto c0 = std::chrono::steady_clock::now();
@@ -702,8 +713,6 @@ extern "C" fdp_status fdp_run_multi_sync(fdp_ctx *c, const fdp_problem *probs, i
   auto t0 = std::chrono::steady_clock::now();
   FDP_CK(cudaSetDevice(c->device), "cudaSetDevice");
   std::vector<MultiPart> parts(static_cast<size_t>(count));
-  uint32_t *pinned = nullptr;
-  cudaEvent_t fork = nullptr;
   cudaGraph_t g = nullptr;
   cudaGraphExec_t ge = nullptr;
   fdp_status rs = FDP_OK;
@@ -711,22 +720,11 @@ extern "C" fdp_status fdp_run_multi_sync(fdp_ctx *c, const fdp_problem *probs, i
   auto cleanup = [&]() {
     if (ge) cudaGraphExecDestroy(ge);
     if (g) cudaGraphDestroy(g);
-    for (size_t i = 0; i < parts.size(); ++i) {
-      MultiPart &p = parts[i];
-      if (p.main) cudaFree(p.main);
-      if (p.blk) cudaFree(p.blk);
-      if (p.esc) cudaFree(p.esc);
-      if (p.acc) cudaFree(p.acc);
-      if (p.res) cudaFree(p.res);
-      if (p.err) cudaFree(p.err);
-      if (p.s) cudaStreamDestroy(p.s);
-      if (p.done) cudaEventDestroy(p.done);
-      if (p.span_s) cudaStreamDestroy(p.span_s);
-      if (p.span_fork) cudaEventDestroy(p.span_fork);
-      if (p.span_join) cudaEventDestroy(p.span_join);
+    if (c->cap_multi > kMultiKeep) {
+      cudaFree(c->d_multi);
+      c->d_multi = nullptr;
+      c->cap_multi = 0;
     }
-    if (pinned) cudaFreeHost(pinned);
-    if (fork) cudaEventDestroy(fork);
   };
 #define MULTI_CK(expr, what)                   \
   do {                                         \
@@ -734,32 +732,81 @@ extern "C" fdp_status fdp_run_multi_sync(fdp_ctx *c, const fdp_problem *probs, i
     if (rs != FDP_OK) { cleanup(); return rs; } \
   } while (0)
   // Residues of every problem, then one error word per problem.
-  MULTI_CK(cudaMallocHost(&pinned, sizeof(uint32_t) * size_t(total_k + count)), "pinned residues");
-  MULTI_CK(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming), "event");
+  if (c->cap_hmulti < size_t(total_k + count)) {
+    if (c->h_multi) cudaFreeHost(c->h_multi);
+    c->h_multi = nullptr;
+    c->cap_hmulti = 0;
+    MULTI_CK(cudaMallocHost(&c->h_multi, sizeof(uint32_t) * size_t(total_k + count)), "pinned residues");
+    c->cap_hmulti = size_t(total_k + count);
+  }
+  uint32_t *const pinned = c->h_multi;
+  // Two streams and three events a problem, and the fork event.
+  while (c->multi_streams.size() < size_t(2 * count)) {
+    cudaStream_t x = nullptr;
+    MULTI_CK(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking), "multi stream");
+    c->multi_streams.push_back(x);
+  }
+  while (c->multi_events.size() < size_t(3 * count + 1)) {
+    cudaEvent_t x = nullptr;
+    MULTI_CK(cudaEventCreateWithFlags(&x, cudaEventDisableTiming), "multi event");
+    c->multi_events.push_back(x);
+  }
+  const cudaEvent_t fork = c->multi_events[size_t(3 * count)];
   for (int i = 0; i < count; ++i) {
     MultiPart &p = parts[size_t(i)];
-    const int W = probs[i].n + 1;
-    if ((rs = fdp_prepare_pass(c, W, &p.t)) != FDP_OK) { cleanup(); return rs; }
+    if ((rs = fdp_prepare_pass(c, probs[i].n + 1, &p.t)) != FDP_OK) { cleanup(); return rs; }
     p.lanes = probs[i].lanes < probs[i].k ? probs[i].lanes : probs[i].k;
-    MULTI_CK(cudaMalloc(&p.main, size_t(fdp::main_states(W)) * p.lanes * 4), "multi main state");
-    MULTI_CK(cudaMalloc(&p.blk, size_t(fdp::blocked_states(W)) * p.lanes * 4 + 4), "multi blocked state");
-    const size_t eb = c->cfg.tail ? size_t(fdp::tail_escape_words(W)) * p.lanes * 4 : 0;
-    size_t free_b = 0, total_b = 0;
-    if (eb && (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b < eb + kEscapeMargin ||
-               cudaMalloc(&p.esc, eb) != cudaSuccess)) {
-      cudaGetLastError();
-      p.esc = nullptr;
-    }
-    MULTI_CK(cudaMalloc(&p.acc, sizeof(unsigned long long) * FDP_MAX_LANES), "multi acc");
-    MULTI_CK(cudaMalloc(&p.res, sizeof(uint32_t) * FDP_MAX_LANES), "multi res");
-    MULTI_CK(cudaMalloc(&p.err, sizeof(unsigned int)), "multi error word");
-    MULTI_CK(cudaStreamCreateWithFlags(&p.s, cudaStreamNonBlocking), "multi stream");
-    MULTI_CK(cudaEventCreateWithFlags(&p.done, cudaEventDisableTiming), "multi event");
+    p.s = c->multi_streams[size_t(2 * i)];
+    p.done = c->multi_events[size_t(3 * i)];
     if (p.lanes > 8) {
-      MULTI_CK(cudaStreamCreateWithFlags(&p.span_s, cudaStreamNonBlocking), "multi stream");
-      MULTI_CK(cudaEventCreateWithFlags(&p.span_fork, cudaEventDisableTiming), "multi event");
-      MULTI_CK(cudaEventCreateWithFlags(&p.span_join, cudaEventDisableTiming), "multi event");
+      p.span_s = c->multi_streams[size_t(2 * i + 1)];
+      p.span_fork = c->multi_events[size_t(3 * i + 1)];
+      p.span_join = c->multi_events[size_t(3 * i + 2)];
     }
+  }
+  // One allocation for every problem's buffers: states, small words and, where
+  // memory allows, the escape words of the fused row tail.
+  auto carve = [&](bool escapes) {
+    size_t at = 0;
+    auto take = [&](size_t bytes) -> char * {
+      char *p = c->d_multi ? c->d_multi + at : nullptr;
+      at += (bytes + 255) / 256 * 256;
+      return p;
+    };
+    for (int i = 0; i < count; ++i) {
+      MultiPart &p = parts[size_t(i)];
+      const int W = probs[i].n + 1;
+      const size_t l4 = size_t(p.lanes) * 4;
+      const bool whole = whole_pass(c, W);
+      p.main = reinterpret_cast<uint32_t *>(take(whole ? 4 : size_t(fdp::main_states(W)) * l4));
+      p.blk = reinterpret_cast<uint32_t *>(take(whole ? 4 : size_t(fdp::blocked_states(W)) * l4 + 4));
+      const size_t eb = escapes && c->cfg.tail ? size_t(fdp::tail_escape_words(W)) * l4 : 0;
+      p.esc = eb ? reinterpret_cast<uint32_t *>(take(eb)) : nullptr;
+      p.acc = reinterpret_cast<unsigned long long *>(take(sizeof(unsigned long long) * FDP_MAX_LANES));
+      p.res = reinterpret_cast<uint32_t *>(take(sizeof(uint32_t) * FDP_MAX_LANES));
+      p.err = reinterpret_cast<unsigned int *>(take(sizeof(unsigned int)));
+    }
+    return at;
+  };
+  for (bool escapes : {true, false}) {
+    const size_t bytes = carve(escapes);
+    if (c->cap_multi < bytes) {
+      if (c->d_multi) cudaFree(c->d_multi);
+      c->d_multi = nullptr;
+      c->cap_multi = 0;
+      size_t free_b = 0, total_b = 0;
+      if (escapes && (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b < bytes + kEscapeMargin)) continue;
+      const cudaError_t e = cudaMalloc(&c->d_multi, bytes);
+      if (e != cudaSuccess && escapes) {
+        cudaGetLastError();
+        c->d_multi = nullptr;
+        continue;
+      }
+      MULTI_CK(e, "multi states");
+      c->cap_multi = bytes;
+    }
+    carve(escapes);
+    break;
   }
   auto c0 = std::chrono::steady_clock::now();
   MULTI_CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal), "begin capture");

@@ -4,6 +4,7 @@
 
 #include <map>
 #include <mutex>
+#include <vector>
 
 #include "../../include/oneesan_fdp.h"
 #include "fdp_launch.h"
@@ -27,6 +28,14 @@ struct fdp_ctx {
   // spans touch disjoint panels, so their cell launches run as two chains.
   cudaStream_t span_stream = nullptr;
   cudaEvent_t span_fork = nullptr, span_join = nullptr;
+  // fdp_run_multi_sync's device memory (kept up to a bound between calls), pinned
+  // results and the streams and events of its problems.
+  char *d_multi = nullptr;
+  size_t cap_multi = 0;
+  uint32_t *h_multi = nullptr;
+  size_t cap_hmulti = 0;  // words
+  std::vector<cudaStream_t> multi_streams;
+  std::vector<cudaEvent_t> multi_events;
   fdp::LaunchCfg cfg;
   std::mutex mu;         // serialises run_sync / apply_cells / time_cells / tuning
   std::mutex tables_mu;  // guards `tables` (also used by the serving thread)
