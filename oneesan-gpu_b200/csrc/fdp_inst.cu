@@ -23,7 +23,7 @@ namespace fdp {
 constexpr int kInstMaxDevices = 64;
 
 struct VariantState {
-  bool limit_set = false;
+  bool limit_set = false, runs_set = false;
   std::map<uint64_t, int> per_sm;  // (block, dynamic shared bytes) -> resident CTAs per SM
 };
 
@@ -34,6 +34,7 @@ cudaError_t launch_cell_t(const CellArgs &a, const LaunchCfg &cfg, cudaStream_t 
   if (cfg.block < 32 || cfg.block > 256 || cfg.block % 32) return cudaErrorInvalidValue;
   if (a.W < 2 || a.W > FDP_MAXW) return cudaErrorInvalidValue;
   const int compact = a.compact == 2 ? 2 : (a.compact && a.lane_items <= FDP_REC_MAX_ITEMS ? 1 : 0);
+  const bool runs = K <= 8 && a.runs != 0 && !a.compact && a.p >= 2;
   const size_t smem = cell_smem_bytes<Idx, K>(cfg.block, a.W, compact, a.lane_items);
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -53,8 +54,19 @@ cudaError_t launch_cell_t(const CellArgs &a, const LaunchCfg &cfg, cudaStream_t 
       if (e != cudaSuccess) return e;
       v.limit_set = true;
     }
-    int &slot = v.per_sm[(uint64_t(a.compact ? 1 : 0) << 62) | (uint64_t(cfg.block) << 32) | uint64_t(smem)];
+    if constexpr (K <= 8) {
+      if (runs && !v.runs_set) {
+        e = cudaFuncSetAttribute(cell_run_kernel<Idx, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(CellSmem<Idx>)));
+        if (e != cudaSuccess) return e;
+        v.runs_set = true;
+      }
+    }
+    int &slot = v.per_sm[(uint64_t(runs ? 2 : (a.compact ? 1 : 0)) << 61) | (uint64_t(cfg.block) << 32) | uint64_t(smem)];
     if (slot == 0) {
+      if constexpr (K <= 8) {
+        if (runs) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&slot, cell_run_kernel<Idx, K>, cfg.block, smem);
+      }
+      if (!runs)
       e = a.compact ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&slot, cell_kernel<Idx, K>, cfg.block, smem)
                     : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&slot, cell_stream_kernel<Idx, K>, cfg.block, smem);
       if (e != cudaSuccess) {
@@ -69,6 +81,12 @@ cudaError_t launch_cell_t(const CellArgs &a, const LaunchCfg &cfg, cudaStream_t 
   const uint64_t per_block = uint64_t(cfg.block) * uint64_t(a.lane_items < 1 ? 1 : a.lane_items);
   const uint64_t need = (a.items + per_block - 1) / per_block;
   if (uint64_t(grid) > need) grid = int(need ? need : 1);
+  if constexpr (K <= 8) {
+    if (runs) {
+      cell_run_kernel<Idx, K><<<grid, cfg.block, smem, s>>>(a);
+      return cudaGetLastError();
+    }
+  }
   if (a.compact) cell_kernel<Idx, K><<<grid, cfg.block, smem, s>>>(a);
   else cell_stream_kernel<Idx, K><<<grid, cfg.block, smem, s>>>(a);
   return cudaGetLastError();

@@ -52,6 +52,7 @@ struct CellArgs {
   int share_prefix;    // decode the prefix a warp chunk shares once per chunk
   int compact;         // small-p cells: 1 = a chunk's items updated grouped by centre type
                        // (lane_items <= FDP_REC_MAX_ITEMS), 2 = grouped with carry-over queues
+  int runs;            // streaming cells: run by run
 };
 
 struct FirstRowArgs {
@@ -292,6 +293,45 @@ FDP_HD Head<Idx> decode_head(const CellArgs &a, const CellSmem<Idx> &sm, const I
   return Head<Idx>{j, r, bm, hw, h, c};
 }
 
+// The RR closures of a c = N head, scanning the high part up.
+template <typename Idx, typename OnCand>
+FDP_HD void for_each_rr(const CellArgs &a, const CellSmem<Idx> &sm, const Head<Idx> &hd, OnCand &&on_cand) {
+  const int p = a.p, h = hd.h;
+  const Idx r = hd.r, bm = hd.bm;
+  // RR closures: every R at depth 1 of the high part (scanning up from p+1),
+  // flipped to L, is a predecessor with pair RR (RV.hpp:70-82).  Its high base
+  // is bm - S0 + S2 + H[q][h], S0/S2 the rank contributions of the positions
+  // below q at their own and at +2 heights.  N symbols are skipped with the
+  // non-N bit mask.
+  const Idx offRR = sm.OFF[h + 2][PR_RR] + r;
+  const uint64_t hw = hd.hw;
+  uint64_t nn = (hw | (hw >> 1)) & 0x5555555555555555ull;
+  Idx S0 = 0, S2 = 0;
+  int ha = h, depth = 1, mx = h;  // mx: highest height below q (the predecessor sits 2 higher)
+  while (nn && depth > 0) {
+#if defined(__CUDA_ARCH__)
+    const int b = __ffsll((long long)nn) - 1;
+#else
+    const int b = __builtin_ctzll(nn);
+#endif
+    nn &= nn - 1;
+    const int q = p + 1 + (b >> 1);
+    if (((hw >> b) & 3u) == SYM_R) {
+      const int hbq = ha + 1;
+      if (depth == 1 && mx + 2 <= a.cap) on_cand(bm - S0 + S2 + sm.H[q][h] + offRR);
+      S0 += sm.H[q][hbq];
+      S2 += sm.H[q][hbq + 2];
+      ha = hbq; ++depth;
+      mx = hbq > mx ? hbq : mx;
+    } else {
+      const int hbq = ha - 1;
+      S0 += sm.H[q][hbq] + (hbq > 0 ? sm.H[q][hbq - 1] : Idx(0));
+      S2 += sm.H[q][hbq + 2] + sm.H[q][hbq + 1];
+      ha = hbq; --depth;
+    }
+  }
+}
+
 // Every closure predecessor (its main index) of a c = N head, handed to
 // on_cand: LL sources scanning the low word down, then RR sources scanning the
 // high part up.
@@ -325,38 +365,7 @@ FDP_HD void for_each_closure(const CellArgs &a, const CellSmem<Idx> &sm, const H
       }
     }
   }
-  // RR closures: every R at depth 1 of the high part (scanning up from p+1),
-  // flipped to L, is a predecessor with pair RR (RV.hpp:70-82).  Its high base
-  // is bm - S0 + S2 + H[q][h], S0/S2 the rank contributions of the positions
-  // below q at their own and at +2 heights.  N symbols are skipped with the
-  // non-N bit mask.
-  const Idx offRR = sm.OFF[h + 2][PR_RR] + r;
-  const uint64_t hw = hd.hw;
-  uint64_t nn = (hw | (hw >> 1)) & 0x5555555555555555ull;
-  Idx S0 = 0, S2 = 0;
-  int ha = h, depth = 1, mx = h;  // mx: highest height below q (the predecessor sits 2 higher)
-  while (nn && depth > 0) {
-#if defined(__CUDA_ARCH__)
-    const int b = __ffsll((long long)nn) - 1;
-#else
-    const int b = __builtin_ctzll(nn);
-#endif
-    nn &= nn - 1;
-    const int q = p + 1 + (b >> 1);
-    if (((hw >> b) & 3u) == SYM_R) {
-      const int hbq = ha + 1;
-      if (depth == 1 && mx + 2 <= a.cap) on_cand(bm - S0 + S2 + sm.H[q][h] + offRR);
-      S0 += sm.H[q][hbq];
-      S2 += sm.H[q][hbq + 2];
-      ha = hbq; ++depth;
-      mx = hbq > mx ? hbq : mx;
-    } else {
-      const int hbq = ha - 1;
-      S0 += sm.H[q][hbq] + (hbq > 0 ? sm.H[q][hbq - 1] : Idx(0));
-      S2 += sm.H[q][hbq + 2] + sm.H[q][hbq + 1];
-      ha = hbq; --depth;
-    }
-  }
+  for_each_rr<Idx>(a, sm, hd, on_cand);
 }
 
 // c = R / L, one span at a time (X = NR/NL, Y = RN/LN):
@@ -645,6 +654,187 @@ FDP_HD void cell_item(const CellArgs &a, const CellSmem<Idx> &sm, const Idx j, c
   const Head<Idx> hd = decode_head<Idx>(a, sm, j, pf);
   if (hd.c != 0) item_x<Idx, K>(a, sm, hd);
   else item_n<Idx, K>(a, sm, hd, cand, cstride);
+}
+
+// ---- runs -------------------------------------------------------------------
+// Consecutive blocked indices with the same high prefix and centre symbol form
+// a run: their words sit side by side, so every word a run's item reads or
+// writes is a base of the run plus the item's offset, except for the LL closures
+// below the low symbols the run shares.  The streaming cells process a warp
+// chunk run by run: one decode and one closure scan for the run, then plain
+// streams.
+#define FDP_RUN_SOURCES 18  // RL and the closures of one word
+
+template <typename Idx>
+struct RunN {
+  Idx rem;         // rank left below `pos` for the run's first item
+  Idx pre2;        // +2-shifted rank of the shared low symbols
+  int pos, hb, depth, mx;  // where the item's own LL scan goes on (depth 0: nowhere)
+  int n;           // sources at list[k] + offset
+};
+
+// The shared sources of the c = N items hd.j .. hd.j + len - 1 (all in hd's run).
+template <typename Idx>
+FDP_HD RunN<Idx> run_sources(const CellArgs &a, const CellSmem<Idx> &sm, const Head<Idx> &hd, Idx len, Idx *list) {
+  const int p = a.p, h = hd.h;
+  RunN<Idx> s{hd.r, Idx(0), p - 2, h, p >= 3 ? 1 : 0, h, 0};
+  if (p >= 2 && h > 0) list[s.n++] = hd.bm + sm.OFF[h][PR_RL] + hd.r;
+  // LL closures in the low symbols the run's first and last item share.
+  if (p >= 3) {
+    const Idx baseLL = hd.bm + sm.OFF[h][PR_LL];
+    Idx r0 = hd.r, r1 = hd.r + (len - 1);
+    for (; s.pos >= 0 && s.depth > 0; --s.pos) {
+      const Idx z0 = sm.H[s.pos][s.hb];
+      const Idx z1 = z0 + (s.hb > 0 ? sm.H[s.pos][s.hb - 1] : Idx(0));
+      const int s0 = r0 >= z1 ? 2 : (r0 >= z0 ? 1 : 0), s1 = r1 >= z1 ? 2 : (r1 >= z0 ? 1 : 0);
+      if (s0 != s1) break;
+      if (s0 == 0) continue;
+      const Idx up2 = sm.H[s.pos][s.hb + 2];
+      if (s0 == 1) {
+        r0 -= z0;
+        r1 -= z0;
+        s.pre2 += up2;
+        --s.depth;
+        --s.hb;
+      } else {
+        r0 -= z1;
+        r1 -= z1;
+        if (s.depth == 1 && s.mx + 2 <= a.cap) list[s.n++] = baseLL + s.pre2 + up2 + r0;
+        s.pre2 += up2 + sm.H[s.pos][s.hb + 1];
+        ++s.depth;
+        ++s.hb;
+        s.mx = s.hb > s.mx ? s.hb : s.mx;
+      }
+    }
+    if (s.pos < 0) s.depth = 0;
+    s.rem = r0;
+  }
+  for_each_rr<Idx>(a, sm, hd, [&](Idx idx) { list[s.n++] = idx; });
+  return s;
+}
+
+// The LL closures of the item at offset o of a run, below the shared symbols.
+template <typename Idx, typename OnCand>
+FDP_HD void run_own_closures(const CellArgs &a, const CellSmem<Idx> &sm, const Head<Idx> &hd, const RunN<Idx> &s, Idx o,
+                             OnCand &&on_cand) {
+  const Idx baseLL = hd.bm + sm.OFF[hd.h][PR_LL];
+  Idx rem = s.rem + o, pre2 = s.pre2;
+  int hb = s.hb, depth = s.depth, mx = s.mx;
+  for (int pos = s.pos; pos >= 0 && depth > 0; --pos) {
+    const Idx z0 = sm.H[pos][hb];
+    if (rem < z0) continue;
+    rem -= z0;
+    const Idx z1 = hb > 0 ? sm.H[pos][hb - 1] : Idx(0);
+    const Idx up2 = sm.H[pos][hb + 2];
+    if (rem < z1) {
+      pre2 += up2;
+      --depth;
+      --hb;
+    } else {
+      rem -= z1;
+      if (depth == 1 && mx + 2 <= a.cap) on_cand(baseLL + pre2 + up2 + rem);
+      pre2 += up2 + sm.H[pos][hb + 1];
+      ++depth;
+      ++hb;
+      mx = hb > mx ? hb : mx;
+    }
+  }
+}
+
+// Items o0, o0 + 32, ... (U of them, those below len) of a c = R/L run, p >= 2.
+template <typename Idx, int K, int U>
+FDP_HD void run_x(const CellArgs &a, Idx iA, Idx iB, Idx j, Idx o0, Idx len) {
+  uint32_t x[U][K], y[U][K], b[U][K];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const Idx o = o0 + Idx(32 * u);
+    if (o < len) {
+      ld_span<K, 0, K>(a.main, a.mstates, size_t(iA + o), x[u]);
+      ld_span<K, 0, K>(a.main, a.mstates, size_t(iB + o), y[u]);
+      if (!a.blk_in_zero) ld_span<K, 0, K>(a.blk, a.items, size_t(j + o), b[u]);
+      else {
+#pragma unroll
+        for (int i = 0; i < K; ++i) b[u][i] = 0;
+      }
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const Idx o = o0 + Idx(32 * u);
+    if (o < len) {
+#pragma unroll
+      for (int i = 0; i < K; ++i) y[u][i] = add_mod(add_mod(x[u][i], y[u][i], a.mod[i]), b[u][i], a.mod[i]);
+      st_span<K, 0, K>(a.main, a.mstates, size_t(iA + o), y[u]);
+      st_span<K, 0, K>(a.blk, a.items, size_t(j + o), x[u]);
+    }
+  }
+}
+
+// The same for a c = N run, p >= 2.
+template <typename Idx, int K, int U>
+FDP_HD void run_n(const CellArgs &a, const CellSmem<Idx> &sm, const Head<Idx> &hd, const RunN<Idx> &s, const Idx *list,
+                  Idx o0, Idx len) {
+  const Idx iNN = hd.bm + sm.OFF[hd.h][PR_NN] + hd.r, iLR = hd.bm + sm.OFF[hd.h][PR_LR] + hd.r;
+  const bool lr = hd.h + 1 <= a.cap;
+  uint32_t x[U][K], y[U][K], b[U][K], acc[U][K];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const Idx o = o0 + Idx(32 * u);
+#pragma unroll
+    for (int i = 0; i < K; ++i) acc[u][i] = b[u][i] = 0;
+    if (o < len) {
+      ld_span<K, 0, K>(a.main, a.mstates, size_t(iNN + o), x[u]);
+      if (!a.blk_in_zero) ld_span<K, 0, K>(a.blk, a.items, size_t(hd.j + o), b[u]);
+      if (lr) ld_span<K, 0, K>(a.main, a.mstates, size_t(iLR + o), y[u]);
+    }
+  }
+  for (int k = 0; k < s.n; ++k) {
+    const Idx base = list[k];
+    uint32_t v[U][K];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (o0 + Idx(32 * u) < len) ld_span<K, 0, K>(a.main, a.mstates, size_t(base + o0 + Idx(32 * u)), v[u]);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int i = 0; i < K; ++i)
+        if (o0 + Idx(32 * u) < len) acc[u][i] = add_mod(acc[u][i], v[u][i], a.mod[i]);
+  }
+  if (s.depth > 0) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const Idx o = o0 + Idx(32 * u);
+      if (o < len)
+        run_own_closures<Idx>(a, sm, hd, s, o, [&](Idx idx) {
+          uint32_t v[K];
+          ld_span<K, 0, K>(a.main, a.mstates, size_t(idx), v);
+#pragma unroll
+          for (int i = 0; i < K; ++i) acc[u][i] = add_mod(acc[u][i], v[i], a.mod[i]);
+        });
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const Idx o = o0 + Idx(32 * u);
+    if (o < len) {
+      if (lr) {
+#pragma unroll
+        for (int i = 0; i < K; ++i) y[u][i] = add_mod(y[u][i], x[u][i], a.mod[i]);
+        st_span<K, 0, K>(a.main, a.mstates, size_t(iLR + o), y[u]);
+      }
+#pragma unroll
+      for (int i = 0; i < K; ++i) x[u][i] = add_mod(x[u][i], b[u][i], a.mod[i]);
+      st_span<K, 0, K>(a.main, a.mstates, size_t(iNN + o), x[u]);
+      st_span<K, 0, K>(a.blk, a.items, size_t(hd.j + o), acc[u]);
+    }
+  }
+}
+
+// Items of a run from its item hd on.
+template <typename Idx>
+FDP_HD Idx run_left(const CellArgs &a, const CellSmem<Idx> &sm, const Head<Idx> &hd) {
+  const int h = hd.h + (hd.c == 1 ? -1 : (hd.c == 2 ? 1 : 0));
+  return sm.H[a.p - 1][h] - hd.r;
 }
 
 // ---- first row ----------------------------------------------------------------

@@ -170,6 +170,46 @@ __global__ void __launch_bounds__(256, stream_min_blocks<K>()) cell_stream_kerne
   cell_body<Idx, K, false>(a);
 }
 
+// The streaming cells of lane counts up to 8, p >= 2, run by run.  Bound at one
+// lane: instruction issue (half the slots busy, of which the chunk's prefix walk
+// and closure scan take most, n = 20: 147 a warp of items, DRAM 2.9 TB/s); at 8
+// lanes: HBM.  Three CTAs per SM: 64 registers spill at most lane counts.
+template <typename Idx, int K>
+__global__ void __launch_bounds__(256, 3) cell_run_kernel(const CellArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ Idx lists[8][FDP_RUN_SOURCES];
+  CellSmem<Idx> &sm = *reinterpret_cast<CellSmem<Idx> *>(smem_raw);
+  load_cell_smem<Idx>(sm, reinterpret_cast<const WidthTables<Idx> *>(a.tables), a.W, a.p);
+  __syncthreads();
+  constexpr int U = K == 1 ? 4 : (K == 2 ? 2 : 1);  // items of a run a lane has in flight together
+  const Idx n = Idx(a.items);
+  const Idx chunk = Idx(32) * Idx(a.lane_items > 0 ? a.lane_items : 1);
+  const Idx wpb = Idx(blockDim.x >> 5);
+  const Idx step = Idx(gridDim.x) * wpb * chunk;
+  const Idx lane = Idx(threadIdx.x & 31);
+  Idx *const list = lists[threadIdx.x >> 5];
+  for (Idx jb = (Idx(blockIdx.x) * wpb + Idx(threadIdx.x >> 5)) * chunk; jb < n; jb += step) {
+    const Idx je = (n - jb > chunk) ? jb + chunk : n;
+    const Prefix<Idx> pf = shared_prefix<Idx>(a, sm, jb, je - 1);
+    for (Idx j = jb; j < je;) {
+      const Head<Idx> hd = decode_head<Idx>(a, sm, j, pf);
+      const Idx left = run_left<Idx>(a, sm, hd), len = left < je - j ? left : je - j;
+      if (hd.c != 0) {
+        Idx ia, ib;
+        x_words<Idx>(sm, hd, ia, ib);
+        for (Idx o = lane; o < len; o += Idx(32 * U)) run_x<Idx, K, U>(a, ia, ib, j, o, len);
+      } else {
+        __syncwarp();
+        const RunN<Idx> s = run_sources<Idx>(a, sm, hd, len, list);  // every lane writes the same list
+        __syncwarp();
+        for (Idx o = lane; o < len; o += Idx(32 * U)) run_n<Idx, K, U>(a, sm, hd, s, list, o, len);
+      }
+      j += len;
+    }
+    if (n - jb <= step) break;  // the next chunk start would be past n (and may wrap)
+  }
+}
+
 template <typename Idx, int K>
 __global__ void __launch_bounds__(256) first_row_init_kernel(const FirstRowArgs a) {
   __shared__ Idx sH[FDP_MAXW + 1][FDP_HT];

@@ -76,11 +76,31 @@ static int run_cells(int W, int cap, uint64_t seed) {
     a.main = gm.data();
     a.blk = gb.data();
     const uint64_t CH = uint64_t(32) * (1 + (seed + uint64_t(p)) % 8);
-    const int mode = int((seed + uint64_t(p)) % 3);  // 0: no sharing; 1: shared, index order; 2: shared, grouped
+    // 0: no sharing; 1: shared, index order; 2: shared, grouped; 3: run by run
+    const int mode = int((seed + uint64_t(p)) % ((K <= 8 && p >= 2) ? 4 : 3));
     for (uint64_t jb = 0; jb < D; jb += CH) {
       const uint64_t jl = std::min(D, jb + CH) - 1;
       const Prefix<Idx> pf = mode ? shared_prefix<Idx>(a, sm, Idx(jb), Idx(jl)) : empty_prefix<Idx>(a);
-      if (mode < 2) {
+      if (mode == 3) {
+        if constexpr (K <= 8) {
+          constexpr int U = K == 1 ? 4 : (K == 3 ? 2 : 1);
+          for (uint64_t j = jb; j <= jl;) {
+            const Head<Idx> hd = decode_head<Idx>(a, sm, Idx(j), pf);
+            const uint64_t left = run_left<Idx>(a, sm, hd), len = std::min<uint64_t>(left, jl + 1 - j);
+            Idx list[FDP_RUN_SOURCES], ia, ib;
+            RunN<Idx> s{};
+            if (hd.c) x_words<Idx>(sm, hd, ia, ib);
+            else s = run_sources<Idx>(a, sm, hd, Idx(len), list);
+            if (!left || s.n > FDP_RUN_SOURCES) { ++bad; break; }
+            for (uint64_t lane = 0; lane < 32; ++lane)
+              for (uint64_t o = lane; o < len; o += 32 * U) {
+                if (hd.c) run_x<Idx, K, U>(a, ia, ib, Idx(j), Idx(o), Idx(len));
+                else run_n<Idx, K, U>(a, sm, hd, s, list, Idx(o), Idx(len));
+              }
+            j += len;
+          }
+        }
+      } else if (mode < 2) {
         for (uint64_t j = jb; j <= jl; ++j) cell_item<Idx, K>(a, sm, Idx(j), pf, cand.data(), 1);
       } else {
         std::vector<Head<Idx>> hx, hn;
