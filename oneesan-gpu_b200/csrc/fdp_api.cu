@@ -21,7 +21,7 @@ static thread_local std::string g_last_error;
 
 // Device memory left free beside an escape buffer.
 static constexpr size_t kEscapeMargin = size_t(1) << 30;
-static constexpr size_t kWindowEscapes = size_t(1) << 30;
+static constexpr size_t kWindowEscapes = size_t(20) << 30;
 // Device memory fdp_run_multi_sync keeps for its next call.
 static constexpr size_t kMultiKeep = size_t(2) << 30;
 
@@ -250,12 +250,18 @@ fdp_status fdp_prepare_pass(fdp_ctx *c, int W, const DevTables **full) {
   return FDP_OK;
 }
 
-static fdp_status ensure_buffer(uint32_t **buf, size_t *cap, size_t bytes, const char *what) {
+static fdp_status ensure_buffer(fdp_ctx *c, uint32_t **buf, size_t *cap, size_t bytes, const char *what) {
   if (*cap >= bytes && *buf) return FDP_OK;
   if (*buf) cudaFree(*buf);
   *buf = nullptr;
   *cap = 0;
-  FDP_CK(cudaMalloc(buf, bytes ? bytes : 4), what);
+  if (cudaMalloc(buf, bytes ? bytes : 4) != cudaSuccess) {  // once more without what the window pool keeps
+    cudaGetLastError();
+    *buf = nullptr;
+    if (c->esc_pool) cudaMemPoolTrimTo(c->esc_pool, 0);
+    c->esc_pool_bytes = 0;
+    FDP_CK(cudaMalloc(buf, bytes ? bytes : 4), what);
+  }
   *cap = bytes;
   return FDP_OK;
 }
@@ -277,8 +283,8 @@ static fdp_status ensure_state(fdp_ctx *c, int W, int lanes, bool want_esc) {
     c->d_multi = nullptr;
     c->cap_multi = 0;
   }
-  fdp_status s = ensure_buffer(&c->d_main, &c->cap_main, mb, "main state");
-  if (s == FDP_OK) s = ensure_buffer(&c->d_blk, &c->cap_blk, bb, "blocked state");
+  fdp_status s = ensure_buffer(c, &c->d_main, &c->cap_main, mb, "main state");
+  if (s == FDP_OK) s = ensure_buffer(c, &c->d_blk, &c->cap_blk, bb, "blocked state");
   if (s != FDP_OK || !eb || c->cap_esc >= eb) return s;
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b > eb + kEscapeMargin &&
@@ -486,11 +492,13 @@ extern "C" fdp_status fdp_run_sync(fdp_ctx *c, const fdp_problem *pr, uint32_t *
 
 // Escape words for one window of fdp_apply_cells, or null: allocated and freed
 // in the order of the caller's stream, so windows on other streams get words of
-// their own.  The pool is the context's and keeps kWindowEscapes bytes between
-// calls; a window that needs more runs cell by cell, as mapping fresh memory
-// for each call costs more than the fused tail gives (15.7 GB at width 24, one
-// lane: a first window 1387 against 857 ms).  So does a stream under capture
-// (the captured work must not depend on an allocation of this context).
+// their own.  The pool is the context's and keeps at most kWindowEscapes bytes
+// for the next window (mapping fresh memory costs more than the fused tail
+// gives: 15.7 GB at width 24, one lane, 0.75 s); it is given back when a state
+// buffer of the context cannot be had, and with the context.  A pool that would
+// have to grow leaves three quarters of what is free to others.  A window that
+// needs more, or a stream under capture (the captured work must not depend on an
+// allocation of this context), runs cell by cell.
 static uint32_t *window_escapes(fdp_ctx *c, int W, int lanes, cudaStream_t st) {
   const size_t bytes = size_t(fdp::tail_escape_words(W)) * lanes * 4;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -510,10 +518,15 @@ static uint32_t *window_escapes(fdp_ctx *c, int W, int lanes, cudaStream_t st) {
     if (ok) cudaMemPoolSetAttribute(c->esc_pool, cudaMemPoolAttrReleaseThreshold, &keep);
     else c->esc_pool = nullptr;
   }
+  if (ok && bytes > c->esc_pool_bytes) {
+    size_t free_b = 0, total_b = 0;
+    ok = cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b / 4 > bytes - c->esc_pool_bytes;
+  }
   if (!ok || cudaMallocFromPoolAsync(&p, bytes, c->esc_pool, st) != cudaSuccess) {
     cudaGetLastError();
     return nullptr;
   }
+  if (bytes > c->esc_pool_bytes) c->esc_pool_bytes = bytes;
   return p;
 }
 

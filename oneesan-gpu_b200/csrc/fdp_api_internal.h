@@ -18,6 +18,7 @@ struct fdp_ctx {
   uint32_t *d_esc = nullptr;             // escape words of the fused row tail (optional)
   size_t cap_main = 0, cap_blk = 0, cap_esc = 0;
   cudaMemPool_t esc_pool = nullptr;      // escape words of fdp_apply_cells, stream-ordered
+  size_t esc_pool_bytes = 0;             // the largest window it has held
   unsigned long long *d_acc = nullptr;   // first-row dot accumulators
   uint32_t *d_res = nullptr;             // residues on the device
   uint32_t *h_res = nullptr;             // residues, pinned host
