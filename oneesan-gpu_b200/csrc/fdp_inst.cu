@@ -81,15 +81,12 @@ cudaError_t launch_cell_t(const CellArgs &a, const LaunchCfg &cfg, cudaStream_t 
   const uint64_t per_block = uint64_t(cfg.block) * uint64_t(a.lane_items < 1 ? 1 : a.lane_items);
   const uint64_t need = (a.items + per_block - 1) / per_block;
   if (uint64_t(grid) > need) grid = int(need ? need : 1);
+  const bool overlap = 4 * grid <= 3 * device_sm_count() * per_sm;
   if constexpr (K <= 8) {
-    if (runs) {
-      cell_run_kernel<Idx, K><<<grid, cfg.block, smem, s>>>(a);
-      return cudaGetLastError();
-    }
+    if (runs) return launch_chained(cell_run_kernel<Idx, K>, unsigned(grid), unsigned(cfg.block), smem, s, a, overlap);
   }
-  if (a.compact) cell_kernel<Idx, K><<<grid, cfg.block, smem, s>>>(a);
-  else cell_stream_kernel<Idx, K><<<grid, cfg.block, smem, s>>>(a);
-  return cudaGetLastError();
+  return a.compact ? launch_chained(cell_kernel<Idx, K>, unsigned(grid), unsigned(cfg.block), smem, s, a, overlap)
+                   : launch_chained(cell_stream_kernel<Idx, K>, unsigned(grid), unsigned(cfg.block), smem, s, a, overlap);
 }
 
 template <typename Idx, int K>

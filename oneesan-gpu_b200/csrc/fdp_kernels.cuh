@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include "fdp_item.cuh"
+#include "fdp_launch.h"
 
 namespace fdp {
 
@@ -56,8 +57,10 @@ __device__ __forceinline__ void cell_body(const CellArgs &a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   CellSmem<Idx> &sm = *reinterpret_cast<CellSmem<Idx> *>(smem_raw);
   Idx *cand = reinterpret_cast<Idx *>(smem_raw + sizeof(CellSmem<Idx>));
+  chain_next();
   load_cell_smem<Idx>(sm, reinterpret_cast<const WidthTables<Idx> *>(a.tables), a.W, a.p);
   __syncthreads();
+  chain_wait();
   // Each warp takes chunks of 32 * lane_items consecutive blocked indices;
   // lane l handles indices l, l + 32, ... of its chunk, so every access of a
   // warp still covers 32 consecutive states.  With share_prefix the top
@@ -179,8 +182,10 @@ __global__ void __launch_bounds__(256, 3) cell_run_kernel(const CellArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ Idx lists[8][FDP_RUN_SOURCES];
   CellSmem<Idx> &sm = *reinterpret_cast<CellSmem<Idx> *>(smem_raw);
+  chain_next();
   load_cell_smem<Idx>(sm, reinterpret_cast<const WidthTables<Idx> *>(a.tables), a.W, a.p);
   __syncthreads();
+  chain_wait();
   constexpr int U = K == 1 ? 4 : (K == 2 ? 2 : 1);  // items of a run a lane has in flight together
   const Idx n = Idx(a.items);
   const Idx chunk = Idx(32) * Idx(a.lane_items > 0 ? a.lane_items : 1);

@@ -84,4 +84,33 @@ cudaError_t launch_ternary_index_chunked(int chunk, const uint32_t *codes, uint3
 
 int device_sm_count();
 
+#if defined(__CUDACC__)
+// Small launches of one chain overlap at their seams: a kernel launched with
+// `overlap` starts once the CTAs of the one before it have all started, if there
+// is room, sets up what no kernel writes (tables), and waits with chain_wait for
+// the one before it to end before it touches a state.  Every CTA of a chained
+// kernel calls both.  The line is a grid of three quarters of the resident CTAs,
+// where the next one's first CTAs find room: width 14 x 16 lanes, cells 13..6,
+// 159 -> 114 us; a full grid's early successors only hold room that its own CTAs
+// and other streams could use (n = 20 x 4 409 -> 458 ms).
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename Kernel, typename Args>
+cudaError_t launch_chained(Kernel kernel, unsigned grid, unsigned block, size_t smem, cudaStream_t s, const Args &args,
+                           bool overlap) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, args);
+}
+#endif
+
 }  // namespace fdp
