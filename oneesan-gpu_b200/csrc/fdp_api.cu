@@ -287,12 +287,36 @@ static fdp_status ensure_state(fdp_ctx *c, int W, int lanes, bool want_esc) {
   if (s == FDP_OK) s = ensure_buffer(c, &c->d_blk, &c->cap_blk, bb, "blocked state");
   if (s != FDP_OK || !eb || c->cap_esc >= eb) return s;
   size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b <= eb + kEscapeMargin &&
+      free_b + (c->cap_main - mb) + (c->cap_blk - bb) > eb + kEscapeMargin) {
+    // The buffers of a larger problem stand in the way: exact ones leave room.
+    cudaFree(c->d_main);
+    cudaFree(c->d_blk);
+    c->d_main = c->d_blk = nullptr;
+    c->cap_main = c->cap_blk = 0;
+    s = ensure_buffer(c, &c->d_main, &c->cap_main, mb, "main state");
+    if (s == FDP_OK) s = ensure_buffer(c, &c->d_blk, &c->cap_blk, bb, "blocked state");
+    if (s != FDP_OK) return s;
+  }
   if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b > eb + kEscapeMargin &&
       cudaMalloc(&c->d_esc, eb) == cudaSuccess)
     c->cap_esc = eb;
   else
     cudaGetLastError();
   return FDP_OK;
+}
+
+// Residues a pass of fdp_run_sync really holds: `lanes`, or one span of 8 where the
+// fused row tail's escape words fit beside 8 lanes but not beside all of them
+// (n = 22, 14 lanes: 16.4 s in one pass of single cells, 13.5 s as passes of 8 and 6).
+static int lanes_with_escapes(const fdp_ctx *c, int W, int lanes) {
+  if (lanes <= 8 || !c->cfg.tail || whole_pass(c, W)) return lanes;
+  const size_t state = size_t(fdp::main_states(W) + fdp::blocked_states(W)) * 4, esc = fdp::tail_escape_words(W) * 4;
+  size_t free_b = 0, total_b = 0;
+  if (!esc || (state + esc) * size_t(lanes) < (size_t(32) << 30) || cudaMemGetInfo(&free_b, &total_b) != cudaSuccess)
+    return lanes;
+  const size_t have = free_b + c->cap_main + c->cap_blk + c->cap_esc + c->cap_multi;
+  return (state + esc) * size_t(lanes) + kEscapeMargin > have && (state + esc) * 8 + kEscapeMargin <= have ? 8 : lanes;
 }
 
 // Enqueue one whole residue pass on `s`: the row-0 state, the row sweeps, the
@@ -439,7 +463,7 @@ extern "C" fdp_status fdp_run_sync(fdp_ctx *c, const fdp_problem *pr, uint32_t *
   const int W = pr->n + 1;
   const DevTables *t = nullptr;
   if ((s = fdp_prepare_pass(c, W, &t)) != FDP_OK) return s;
-  const int lanes = pr->lanes < pr->k ? pr->lanes : pr->k;
+  const int lanes = lanes_with_escapes(c, W, pr->lanes < pr->k ? pr->lanes : pr->k);
   if (!whole_pass(c, W) && (s = ensure_state(c, W, lanes, c->cfg.tail)) != FDP_OK) return s;
   // Every pass (lanes residues each) is captured into ONE graph, run with one launch.
   fdp_run_stats acc{};
@@ -496,7 +520,7 @@ extern "C" fdp_status fdp_run_sync(fdp_ctx *c, const fdp_problem *pr, uint32_t *
 // for the next window (mapping fresh memory costs more than the fused tail
 // gives: 15.7 GB at width 24, one lane, 0.75 s); it is given back when a state
 // buffer of the context cannot be had, and with the context.  A pool that would
-// have to grow leaves three quarters of what is free to others.  A window that
+// have to grow leaves at least half of what is free to others.  A window that
 // needs more, or a stream under capture (the captured work must not depend on an
 // allocation of this context), runs cell by cell.
 static uint32_t *window_escapes(fdp_ctx *c, int W, int lanes, cudaStream_t st) {
@@ -520,7 +544,7 @@ static uint32_t *window_escapes(fdp_ctx *c, int W, int lanes, cudaStream_t st) {
   }
   if (ok && bytes > c->esc_pool_bytes) {
     size_t free_b = 0, total_b = 0;
-    ok = cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b / 4 > bytes - c->esc_pool_bytes;
+    ok = cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b / 2 > bytes - c->esc_pool_bytes;
   }
   if (!ok || cudaMallocFromPoolAsync(&p, bytes, c->esc_pool, st) != cudaSuccess) {
     cudaGetLastError();
