@@ -363,9 +363,9 @@ fdp_status fdp_factor_map_apply(fdp_ctx *ctx, const fdp_factor_map *map, uint32_
 void fdp_factor_map_destroy(fdp_factor_map *map);
 
 /*
- * Two consecutive cells p, p-1 fused by recursive pull, out of place, without
- * storing the intermediate vector or a matrix (the reverse2 kernels,
- * R2.cu:1116-1155).  Same result as fdp_apply_cells(p, p-1).
+ * Two consecutive cells p, p-1 out of place, without a matrix (the reverse2
+ * kernels, R2.cu:1116-1155).  Same result as fdp_apply_cells(p, p-1); the
+ * outputs hold the intermediate vector meanwhile.
  */
 fdp_status fdp_reverse2_apply(fdp_ctx *ctx, int width, int p, int lanes, const uint32_t *moduli,
                               const uint32_t *d_in_main, const uint32_t *d_in_block, uint32_t *d_out_main,
