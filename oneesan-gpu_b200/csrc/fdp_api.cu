@@ -19,11 +19,12 @@ static thread_local std::string g_last_error;
 
 #define FDP_RUN_MAX_MODULI 64
 
-// Device memory left free beside an escape buffer.
+// Device memory a synchronous call leaves free beside its escape words.
 static constexpr size_t kEscapeMargin = size_t(1) << 30;
-static constexpr size_t kWindowEscapes = size_t(20) << 30;
-// Device memory fdp_run_multi_sync keeps for its next call.
-static constexpr size_t kMultiKeep = size_t(2) << 30;
+// Device memory the windows' pool keeps mapped, and the most that a synchronous
+// call leaves behind, for the next one.
+static constexpr size_t kPoolKeep = size_t(20) << 30;
+static constexpr size_t kSideKeep = size_t(4) << 30;
 
 static fdp_status cuda_status(cudaError_t e, const char *what) {
   if (e == cudaSuccess) return FDP_OK;
@@ -160,8 +161,7 @@ fdp_ctx::~fdp_ctx() {
   for (auto &kv : tables) fdp::free_tables(&kv.second);
   if (d_main) cudaFree(d_main);
   if (d_blk) cudaFree(d_blk);
-  if (d_esc) cudaFree(d_esc);
-  if (d_multi) cudaFree(d_multi);
+  if (d_side) cudaFree(d_side);
   if (h_multi) cudaFreeHost(h_multi);
   for (cudaStream_t x : multi_streams) cudaStreamDestroy(x);
   for (cudaEvent_t x : multi_events) cudaEventDestroy(x);
@@ -174,7 +174,7 @@ fdp_ctx::~fdp_ctx() {
   if (ev1) cudaEventDestroy(ev1);
   if (span_fork) cudaEventDestroy(span_fork);
   if (span_join) cudaEventDestroy(span_join);
-  if (esc_pool) cudaMemPoolDestroy(esc_pool);
+  if (pool) cudaMemPoolDestroy(pool);
   if (span_stream) cudaStreamDestroy(span_stream);
   if (stream) cudaStreamDestroy(stream);
 }
@@ -250,60 +250,122 @@ fdp_status fdp_prepare_pass(fdp_ctx *c, int W, const DevTables **full) {
   return FDP_OK;
 }
 
+// cudaMalloc for what a call cannot do without: where it fails, once more after
+// the windows in flight have handed their words back and without what the context
+// keeps for later calls.
+cudaError_t fdp_ctx_malloc(fdp_ctx *c, void **p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaErrorMemoryAllocation || (!c->pool && !c->d_side)) return e;
+  cudaGetLastError();
+  if ((e = cudaDeviceSynchronize()) != cudaSuccess) return e;
+  if (c->pool) cudaMemPoolTrimTo(c->pool, 0);
+  if (c->d_side) cudaFree(c->d_side);
+  c->d_side = nullptr;
+  c->cap_side = 0;
+  return cudaMalloc(p, bytes);
+}
+
+// The pool of the windows' escape words, kept mapped up to kPoolKeep bytes.  What
+// lies idle in it stands in nobody's way: cudaMalloc of this process gets it from
+// the driver.
+static cudaError_t pool_take(fdp_ctx *c, void **p, size_t bytes, cudaStream_t st) {
+  if (!c->pool) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = c->device;
+    uint64_t keep = kPoolKeep;
+    cudaError_t e = cudaMemPoolCreate(&c->pool, &props);
+    if (e != cudaSuccess) {
+      c->pool = nullptr;
+      return e;
+    }
+    cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  }
+  return cudaMallocFromPoolAsync(p, bytes, c->pool, st);
+}
+
+// Bytes the pool holds mapped and nobody uses.
+static size_t pool_idle(const fdp_ctx *c) {
+  uint64_t mapped = 0, used = 0;
+  if (!c->pool || cudaMemPoolGetAttribute(c->pool, cudaMemPoolAttrReservedMemCurrent, &mapped) != cudaSuccess ||
+      cudaMemPoolGetAttribute(c->pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
+    return 0;
+  return mapped > used ? size_t(mapped - used) : 0;
+}
+
+// Device memory that one synchronous call (the context locked) takes beside its
+// state.  Up to kSideKeep bytes stay with the context for the next such call; more
+// is freed at the call's end, or no other allocator could have it: with its
+// cudaMalloc that costs 1.7 ms for 1 GiB, 10 ms for 10 GiB and 30 ms for 40 GiB, 0.7
+// % of a pass that needs so much (n = 20, 14 lanes: 1373 -> 1383 ms).
+struct SideMemory {
+  fdp_ctx *c;
+  char *p = nullptr;
+  explicit SideMemory(fdp_ctx *ctx) : c(ctx) {}
+  SideMemory(const SideMemory &) = delete;
+  SideMemory &operator=(const SideMemory &) = delete;
+  ~SideMemory() {
+    if (c->cap_side > kSideKeep) drop();
+  }
+  void drop() {
+    if (c->d_side) cudaFree(c->d_side);
+    c->d_side = nullptr;
+    c->cap_side = 0;
+  }
+  cudaError_t take(size_t bytes) {
+    if (c->cap_side < bytes) {
+      drop();
+      void *q = nullptr;
+      const cudaError_t e = fdp_ctx_malloc(c, &q, bytes);
+      if (e != cudaSuccess) return e;
+      c->d_side = static_cast<char *>(q);
+      c->cap_side = bytes;
+    }
+    p = c->d_side;
+    return cudaSuccess;
+  }
+  // Bytes the call can do without: p stays null unless `leave` bytes remain free.
+  bool take_optional(size_t bytes, size_t leave) {
+    size_t free_b = 0, total_b = 0;
+    if ((c->cap_side >= bytes || (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
+                                  free_b + c->cap_side + pool_idle(c) > bytes + leave)) &&
+        take(bytes) == cudaSuccess)
+      return true;
+    cudaGetLastError();
+    return false;
+  }
+};
+
 static fdp_status ensure_buffer(fdp_ctx *c, uint32_t **buf, size_t *cap, size_t bytes, const char *what) {
   if (*cap >= bytes && *buf) return FDP_OK;
   if (*buf) cudaFree(*buf);
   *buf = nullptr;
   *cap = 0;
-  if (cudaMalloc(buf, bytes ? bytes : 4) != cudaSuccess) {  // once more without what the window pool keeps
-    cudaGetLastError();
-    *buf = nullptr;
-    if (c->esc_pool) cudaMemPoolTrimTo(c->esc_pool, 0);
-    c->esc_pool_bytes = 0;
-    FDP_CK(cudaMalloc(buf, bytes ? bytes : 4), what);
-  }
+  FDP_CK(fdp_ctx_malloc(c, reinterpret_cast<void **>(buf), bytes ? bytes : 4), what);
   *cap = bytes;
   return FDP_OK;
 }
 
-// The context's state buffers for `lanes` lanes of width W, and, where
-// `want_esc` and device memory allow, the escape words of the fused row tail.
-// Those are optional: they go first when a state buffer has to grow, and a
-// pass without them runs every cell as its own launch.
-static fdp_status ensure_state(fdp_ctx *c, int W, int lanes, bool want_esc) {
+// The context's state buffers for `lanes` lanes of width W.  Where a call that
+// also wants `beside` bytes could have them but for the buffers of a larger
+// problem, exact buffers take their place.
+static fdp_status ensure_state(fdp_ctx *c, int W, int lanes, size_t beside) {
   const size_t mb = size_t(fdp::main_states(W)) * lanes * 4, bb = size_t(fdp::blocked_states(W)) * lanes * 4;
-  const size_t eb = want_esc ? size_t(fdp::tail_escape_words(W)) * lanes * 4 : 0;
-  if (c->d_esc && (c->cap_main < mb || c->cap_blk < bb || c->cap_esc < eb)) {
-    cudaFree(c->d_esc);
-    c->d_esc = nullptr;
-    c->cap_esc = 0;
-  }
-  if (c->d_multi && (c->cap_main < mb || c->cap_blk < bb)) {
-    cudaFree(c->d_multi);
-    c->d_multi = nullptr;
-    c->cap_multi = 0;
+  size_t free_b = 0, total_b = 0;
+  if (beside > c->cap_side && c->cap_main >= mb && c->cap_blk >= bb && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
+    free_b += c->cap_side + pool_idle(c);
+    if (free_b <= beside + kEscapeMargin &&
+        free_b + (c->cap_main - mb) + (c->cap_blk - bb) > beside + kEscapeMargin) {
+      cudaFree(c->d_main);
+      cudaFree(c->d_blk);
+      c->d_main = c->d_blk = nullptr;
+      c->cap_main = c->cap_blk = 0;
+    }
   }
   fdp_status s = ensure_buffer(c, &c->d_main, &c->cap_main, mb, "main state");
   if (s == FDP_OK) s = ensure_buffer(c, &c->d_blk, &c->cap_blk, bb, "blocked state");
-  if (s != FDP_OK || !eb || c->cap_esc >= eb) return s;
-  size_t free_b = 0, total_b = 0;
-  if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b <= eb + kEscapeMargin &&
-      free_b + (c->cap_main - mb) + (c->cap_blk - bb) > eb + kEscapeMargin) {
-    // The buffers of a larger problem stand in the way: exact ones leave room.
-    cudaFree(c->d_main);
-    cudaFree(c->d_blk);
-    c->d_main = c->d_blk = nullptr;
-    c->cap_main = c->cap_blk = 0;
-    s = ensure_buffer(c, &c->d_main, &c->cap_main, mb, "main state");
-    if (s == FDP_OK) s = ensure_buffer(c, &c->d_blk, &c->cap_blk, bb, "blocked state");
-    if (s != FDP_OK) return s;
-  }
-  if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b > eb + kEscapeMargin &&
-      cudaMalloc(&c->d_esc, eb) == cudaSuccess)
-    c->cap_esc = eb;
-  else
-    cudaGetLastError();
-  return FDP_OK;
+  return s;
 }
 
 // Residues a pass of fdp_run_sync really holds: `lanes`, or one span of 8 where the
@@ -315,7 +377,7 @@ static int lanes_with_escapes(const fdp_ctx *c, int W, int lanes) {
   size_t free_b = 0, total_b = 0;
   if (!esc || (state + esc) * size_t(lanes) < (size_t(32) << 30) || cudaMemGetInfo(&free_b, &total_b) != cudaSuccess)
     return lanes;
-  const size_t have = free_b + c->cap_main + c->cap_blk + c->cap_esc + c->cap_multi;
+  const size_t have = free_b + pool_idle(c) + c->cap_side + c->cap_main + c->cap_blk;
   return (state + esc) * size_t(lanes) + kEscapeMargin > have && (state + esc) * 8 + kEscapeMargin <= have ? 8 : lanes;
 }
 
@@ -464,7 +526,14 @@ extern "C" fdp_status fdp_run_sync(fdp_ctx *c, const fdp_problem *pr, uint32_t *
   const DevTables *t = nullptr;
   if ((s = fdp_prepare_pass(c, W, &t)) != FDP_OK) return s;
   const int lanes = lanes_with_escapes(c, W, pr->lanes < pr->k ? pr->lanes : pr->k);
-  if (!whole_pass(c, W) && (s = ensure_state(c, W, lanes, c->cfg.tail)) != FDP_OK) return s;
+  // The state, and, where memory allows, the escape words of the fused row tail;
+  // a pass without them runs every cell as its own launch.
+  SideMemory esc(c);
+  if (!whole_pass(c, W)) {
+    const size_t eb = c->cfg.tail ? size_t(fdp::tail_escape_words(W)) * lanes * 4 : 0;
+    if ((s = ensure_state(c, W, lanes, eb)) != FDP_OK) return s;
+    if (eb) esc.take_optional(eb, kEscapeMargin);
+  }
   // Every pass (lanes residues each) is captured into ONE graph, run with one launch.
   fdp_run_stats acc{};
   auto c0 = std::chrono::steady_clock::now();
@@ -475,8 +544,8 @@ extern "C" fdp_status fdp_run_sync(fdp_ctx *c, const fdp_problem *pr, uint32_t *
   fdp_status es = cuda_status(fdp_enqueue_err_reset(c->d_err, c->stream), "error word");
   for (int done = 0; done < pr->k && es == FDP_OK; done += lanes) {
     const int L = (pr->k - done) < lanes ? (pr->k - done) : lanes;
-    es = fdp_enqueue_pass(c, *t, L, pr->moduli + done, c->d_main, c->d_blk, c->d_esc, c->d_acc, c->d_res, c->h_res + done,
-                          c->d_err, c->stream, &launches, c->span_stream, c->span_fork, c->span_join);
+    es = fdp_enqueue_pass(c, *t, L, pr->moduli + done, c->d_main, c->d_blk, reinterpret_cast<uint32_t *>(esc.p),
+                          c->d_acc, c->d_res, c->h_res + done, c->d_err, c->stream, &launches, c->span_stream, c->span_fork, c->span_join);
   }
   if (es == FDP_OK) es = cuda_status(fdp_enqueue_err_read(c->h_err, c->d_err, c->stream), "error word");
   cudaError_t ce = cudaStreamEndCapture(c->stream, &g);
@@ -516,42 +585,30 @@ extern "C" fdp_status fdp_run_sync(fdp_ctx *c, const fdp_problem *pr, uint32_t *
 
 // Escape words for one window of fdp_apply_cells, or null: allocated and freed
 // in the order of the caller's stream, so windows on other streams get words of
-// their own.  The pool is the context's and keeps at most kWindowEscapes bytes
-// for the next window (mapping fresh memory costs more than the fused tail
-// gives: 15.7 GB at width 24, one lane, 0.75 s); it is given back when a state
-// buffer of the context cannot be had, and with the context.  A pool that would
-// have to grow leaves at least half of what is free to others.  A window that
-// needs more, or a stream under capture (the captured work must not depend on an
-// allocation of this context), runs cell by cell.
+// their own.  A pool that would have to grow leaves at least half of what is free
+// to others.  A window that needs more than the pool keeps (mapping fresh memory
+// for each window costs more than the fused tail gives), or a stream under capture
+// (the captured work must not depend on an allocation of this context), runs cell
+// by cell.
 static uint32_t *window_escapes(fdp_ctx *c, int W, int lanes, cudaStream_t st) {
   const size_t bytes = size_t(fdp::tail_escape_words(W)) * lanes * 4;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (!bytes || bytes > kWindowEscapes || !c->cfg.tail || cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+  if (!bytes || bytes > kPoolKeep || !c->cfg.tail || cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
     cudaGetLastError();
     return nullptr;
   }
-  uint32_t *p = nullptr;
+  void *p = nullptr;
   bool ok = fdp::prepare_tail(W) == cudaSuccess;
-  if (ok && !c->esc_pool) {
-    cudaMemPoolProps props{};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = c->device;
-    uint64_t keep = kWindowEscapes;
-    ok = cudaMemPoolCreate(&c->esc_pool, &props) == cudaSuccess;
-    if (ok) cudaMemPoolSetAttribute(c->esc_pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    else c->esc_pool = nullptr;
-  }
-  if (ok && bytes > c->esc_pool_bytes) {
+  const size_t idle = pool_idle(c);
+  if (ok && bytes > idle) {
     size_t free_b = 0, total_b = 0;
-    ok = cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b / 2 > bytes - c->esc_pool_bytes;
+    ok = cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b / 2 > bytes - idle;
   }
-  if (!ok || cudaMallocFromPoolAsync(&p, bytes, c->esc_pool, st) != cudaSuccess) {
+  if (!ok || pool_take(c, &p, bytes, st) != cudaSuccess) {
     cudaGetLastError();
     return nullptr;
   }
-  if (bytes > c->esc_pool_bytes) c->esc_pool_bytes = bytes;
-  return p;
+  return static_cast<uint32_t *>(p);
 }
 
 extern "C" fdp_status fdp_apply_cells(fdp_ctx *c, int width, int p_hi, int p_lo, int lanes, const uint32_t *moduli,
@@ -641,7 +698,7 @@ extern "C" fdp_status fdp_time_cells(fdp_ctx *c, const fdp_problem *pr, int rows
   const DevTables *t = nullptr;
   if ((s = fdp_ctx_tables(c, W, &t)) != FDP_OK) return s;
   const int L = pr->lanes < pr->k ? pr->lanes : pr->k;
-  if ((s = ensure_state(c, W, L, false)) != FDP_OK) return s;
+  if ((s = ensure_state(c, W, L, 0)) != FDP_OK) return s;
   std::vector<cudaEvent_t> ev(size_t(rows) * W * 2);
   for (auto &e : ev) FDP_CK(cudaEventCreate(&e), "event");
   // One untimed launch first: the first launch of a kernel variant also loads
@@ -750,6 +807,7 @@ extern "C" fdp_status fdp_run_multi_sync(fdp_ctx *c, const fdp_problem *probs, i
   auto t0 = std::chrono::steady_clock::now();
   FDP_CK(cudaSetDevice(c->device), "cudaSetDevice");
   std::vector<MultiPart> parts(static_cast<size_t>(count));
+  SideMemory mem(c);
   cudaGraph_t g = nullptr;
   cudaGraphExec_t ge = nullptr;
   fdp_status rs = FDP_OK;
@@ -757,11 +815,6 @@ extern "C" fdp_status fdp_run_multi_sync(fdp_ctx *c, const fdp_problem *probs, i
   auto cleanup = [&]() {
     if (ge) cudaGraphExecDestroy(ge);
     if (g) cudaGraphDestroy(g);
-    if (c->cap_multi > kMultiKeep) {
-      cudaFree(c->d_multi);
-      c->d_multi = nullptr;
-      c->cap_multi = 0;
-    }
   };
 #define MULTI_CK(expr, what)                   \
   do {                                         \
@@ -806,7 +859,7 @@ extern "C" fdp_status fdp_run_multi_sync(fdp_ctx *c, const fdp_problem *probs, i
   auto carve = [&](bool escapes) {
     size_t at = 0;
     auto take = [&](size_t bytes) -> char * {
-      char *p = c->d_multi ? c->d_multi + at : nullptr;
+      char *p = mem.p ? mem.p + at : nullptr;
       at += (bytes + 255) / 256 * 256;
       return p;
     };
@@ -825,26 +878,9 @@ extern "C" fdp_status fdp_run_multi_sync(fdp_ctx *c, const fdp_problem *probs, i
     }
     return at;
   };
-  for (bool escapes : {true, false}) {
-    const size_t bytes = carve(escapes);
-    if (c->cap_multi < bytes) {
-      if (c->d_multi) cudaFree(c->d_multi);
-      c->d_multi = nullptr;
-      c->cap_multi = 0;
-      size_t free_b = 0, total_b = 0;
-      if (escapes && (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b < bytes + kEscapeMargin)) continue;
-      const cudaError_t e = cudaMalloc(&c->d_multi, bytes);
-      if (e != cudaSuccess && escapes) {
-        cudaGetLastError();
-        c->d_multi = nullptr;
-        continue;
-      }
-      MULTI_CK(e, "multi states");
-      c->cap_multi = bytes;
-    }
-    carve(escapes);
-    break;
-  }
+  const bool escapes = mem.take_optional(carve(true), kEscapeMargin);
+  if (!escapes) MULTI_CK(mem.take(carve(false)), "multi states");
+  carve(escapes);
   auto c0 = std::chrono::steady_clock::now();
   MULTI_CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
   cudaEventRecord(fork, c->stream);

@@ -15,10 +15,9 @@ struct fdp_ctx {
   std::map<int, fdp::DevTables> tables;  // per frontier width
   uint32_t *d_main = nullptr;            // run_sync state, [M][lanes]
   uint32_t *d_blk = nullptr;             // run_sync state, [D][lanes]
-  uint32_t *d_esc = nullptr;             // escape words of the fused row tail (optional)
-  size_t cap_main = 0, cap_blk = 0, cap_esc = 0;
-  cudaMemPool_t esc_pool = nullptr;      // escape words of fdp_apply_cells, stream-ordered
-  size_t esc_pool_bytes = 0;             // the largest window it has held
+  char *d_side = nullptr;                // what a synchronous call takes beside its state
+  size_t cap_main = 0, cap_blk = 0, cap_side = 0;
+  cudaMemPool_t pool = nullptr;          // escape words of fdp_apply_cells, stream-ordered
   unsigned long long *d_acc = nullptr;   // first-row dot accumulators
   uint32_t *d_res = nullptr;             // residues on the device
   uint32_t *h_res = nullptr;             // residues, pinned host
@@ -29,10 +28,7 @@ struct fdp_ctx {
   // spans touch disjoint panels, so their cell launches run as two chains.
   cudaStream_t span_stream = nullptr;
   cudaEvent_t span_fork = nullptr, span_join = nullptr;
-  // fdp_run_multi_sync's device memory (kept up to a bound between calls), pinned
-  // results and the streams and events of its problems.
-  char *d_multi = nullptr;
-  size_t cap_multi = 0;
+  // fdp_run_multi_sync's pinned results and the streams and events of its problems.
   uint32_t *h_multi = nullptr;
   size_t cap_hmulti = 0;  // words
   std::vector<cudaStream_t> multi_streams;
@@ -46,6 +42,7 @@ struct fdp_ctx {
 
 fdp_status fdp_ctx_tables(fdp_ctx *c, int W, const fdp::DevTables **out);
 fdp_status fdp_ctx_tables_cap(fdp_ctx *c, int W, int cap, const fdp::DevTables **out);
+cudaError_t fdp_ctx_malloc(fdp_ctx *c, void **p, size_t bytes);
 fdp_status fdp_prepare_pass(fdp_ctx *c, int W, const fdp::DevTables **full);
 // One residue pass of L lanes on stream s.  esc: fdp::tail_escape_words(W) x L
 // words for the fused row tail, or null to run every cell as its own launch.  With span_stream (and fork /

@@ -357,7 +357,7 @@ extern "C" fdp_status fdp_server_start(fdp_ctx *c, const fdp_server_config *cfg)
   sv->ctx = c;
   sv->cfg = *cfg;
   if (sv->cfg.max_bypass_s <= 0) sv->cfg.max_bypass_s = 30.0;
-  e = cudaMalloc(&sv->pool, cfg->hbm_budget_bytes);
+  e = fdp_ctx_malloc(c, reinterpret_cast<void **>(&sv->pool), cfg->hbm_budget_bytes);
   if (e != cudaSuccess) {
     cudaGetLastError();
     fdp_set_last_error("server: cannot reserve the HBM budget");

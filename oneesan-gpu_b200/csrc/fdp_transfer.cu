@@ -474,8 +474,9 @@ fdp_status build_csr(fdp_ctx *c, const SpaceArgs &sa, ull M, ull total, int widt
     if (columns) cudaFree(columns);
     return fdp_cuda_status(ce, what);
   };
-  if ((e = cudaMalloc(&offsets, sizeof(ull) * (total + 1))) != cudaSuccess) return fail(e, "csr offsets");
-  if ((e = cudaMalloc(&err, sizeof(ull))) != cudaSuccess) return fail(e, "csr errors");
+  auto alloc = [&](auto **q, size_t bytes) { return fdp_ctx_malloc(c, reinterpret_cast<void **>(q), bytes); };
+  if ((e = alloc(&offsets, sizeof(ull) * (total + 1))) != cudaSuccess) return fail(e, "csr offsets");
+  if ((e = alloc(&err, sizeof(ull))) != cudaSuccess) return fail(e, "csr errors");
   csr_count_kernel<Group><<<grid_for(total), 256, 0, c->stream>>>(sa, M, total, width, p, paired, offsets);
   if ((e = cudaGetLastError()) != cudaSuccess) return fail(e, "csr count");
   std::vector<ull> off(total + 1);
@@ -493,7 +494,7 @@ fdp_status build_csr(fdp_ctx *c, const SpaceArgs &sa, ull M, ull total, int widt
   if ((e = cudaMemcpyAsync(offsets, off.data(), sizeof(ull) * (total + 1), cudaMemcpyHostToDevice, c->stream)) !=
       cudaSuccess)
     return fail(e, "csr offsets copy");
-  if ((e = cudaMalloc(&columns, sizeof(uint32_t) * (run ? run : 1))) != cudaSuccess) return fail(e, "csr columns");
+  if ((e = alloc(&columns, sizeof(uint32_t) * (run ? run : 1))) != cudaSuccess) return fail(e, "csr columns");
   if ((e = cudaMemsetAsync(err, 0, sizeof(ull), c->stream)) != cudaSuccess) return fail(e, "csr errors");
   csr_fill_kernel<Group><<<grid_for(total), 256, 0, c->stream>>>(sa, M, total, width, p, paired, offsets, columns,
                                                                  err);
@@ -855,11 +856,12 @@ extern "C" fdp_status fdp_factor_map_build(fdp_ctx *c, int width, int p, int pai
   map->gm = gm;
   map->gd = gd;
   const size_t cells = size_t(total) * size_t(max_groups);
-  if ((e = cudaMalloc(&map->gcounts, sizeof(Counts))) != cudaSuccess ||
+  auto alloc = [&](auto **q, size_t bytes) { return fdp_ctx_malloc(c, reinterpret_cast<void **>(q), bytes); };
+  if ((e = alloc(&map->gcounts, sizeof(Counts))) != cudaSuccess ||
       (e = cudaMemcpy(map->gcounts, &hg, sizeof(Counts), cudaMemcpyHostToDevice)) != cudaSuccess ||
-      (e = cudaMalloc(&map->arena_in, sizeof(uint32_t) * cells)) != cudaSuccess ||
-      (e = cudaMalloc(&map->arena_out, sizeof(uint32_t) * cells)) != cudaSuccess ||
-      (e = cudaMalloc(&map->ranks, sizeof(ull) * cells)) != cudaSuccess)
+      (e = alloc(&map->arena_in, sizeof(uint32_t) * cells)) != cudaSuccess ||
+      (e = alloc(&map->arena_out, sizeof(uint32_t) * cells)) != cudaSuccess ||
+      (e = alloc(&map->ranks, sizeof(ull) * cells)) != cudaSuccess)
     return fdp_cuda_status(e, "factor map buffers");
   for (cudaEvent_t &ev : map->ev)
     if ((e = cudaEventCreate(&ev)) != cudaSuccess) return fdp_cuda_status(e, "factor map events");
