@@ -25,6 +25,8 @@ static constexpr size_t kEscapeMargin = size_t(1) << 30;
 // call leaves behind, for the next one.
 static constexpr size_t kPoolKeep = size_t(20) << 30;
 static constexpr size_t kSideKeep = size_t(4) << 30;
+// Windows of a context that hold pool memory at a time.
+static constexpr size_t kWindows = 64;
 
 static fdp_status cuda_status(cudaError_t e, const char *what) {
   if (e == cudaSuccess) return FDP_OK;
@@ -174,6 +176,7 @@ fdp_ctx::~fdp_ctx() {
   if (ev1) cudaEventDestroy(ev1);
   if (span_fork) cudaEventDestroy(span_fork);
   if (span_join) cudaEventDestroy(span_join);
+  for (WindowUse &w : windows) cudaEventDestroy(w.done);
   if (pool) cudaMemPoolDestroy(pool);
   if (span_stream) cudaStreamDestroy(span_stream);
   if (stream) cudaStreamDestroy(stream);
@@ -275,22 +278,38 @@ static cudaError_t pool_take(fdp_ctx *c, void **p, size_t bytes, cudaStream_t st
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = c->device;
     uint64_t keep = kPoolKeep;
+    int off = 0;  // a window never waits for another stream's to get its words
     cudaError_t e = cudaMemPoolCreate(&c->pool, &props);
     if (e != cudaSuccess) {
       c->pool = nullptr;
       return e;
     }
     cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    cudaMemPoolSetAttribute(c->pool, cudaMemPoolReuseAllowInternalDependencies, &off);
   }
   return cudaMallocFromPoolAsync(p, bytes, c->pool, st);
 }
 
-// Bytes the pool holds mapped and nobody uses.
-static size_t pool_idle(const fdp_ctx *c) {
+// Bytes the pool holds mapped that stream st can have.  The pool counts a window's
+// words as unused from the call that frees them on; until its stream gets there
+// they serve that stream alone.
+static size_t pool_idle(fdp_ctx *c, cudaStream_t st) {
   uint64_t mapped = 0, used = 0;
   if (!c->pool || cudaMemPoolGetAttribute(c->pool, cudaMemPoolAttrReservedMemCurrent, &mapped) != cudaSuccess ||
       cudaMemPoolGetAttribute(c->pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
     return 0;
+  for (size_t i = 0; i < c->windows.size();) {
+    WindowUse &w = c->windows[i];
+    if (cudaEventQuery(w.done) == cudaErrorNotReady) {
+      cudaGetLastError();
+      if (w.stream != st) used += w.bytes;
+      ++i;
+    } else {
+      cudaEventDestroy(w.done);
+      w = c->windows.back();
+      c->windows.pop_back();
+    }
+  }
   return mapped > used ? size_t(mapped - used) : 0;
 }
 
@@ -329,7 +348,7 @@ struct SideMemory {
   bool take_optional(size_t bytes, size_t leave) {
     size_t free_b = 0, total_b = 0;
     if ((c->cap_side >= bytes || (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
-                                  free_b + c->cap_side + pool_idle(c) > bytes + leave)) &&
+                                  free_b + c->cap_side + pool_idle(c, c->stream) > bytes + leave)) &&
         take(bytes) == cudaSuccess)
       return true;
     cudaGetLastError();
@@ -354,7 +373,7 @@ static fdp_status ensure_state(fdp_ctx *c, int W, int lanes, size_t beside) {
   const size_t mb = size_t(fdp::main_states(W)) * lanes * 4, bb = size_t(fdp::blocked_states(W)) * lanes * 4;
   size_t free_b = 0, total_b = 0;
   if (beside > c->cap_side && c->cap_main >= mb && c->cap_blk >= bb && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
-    free_b += c->cap_side + pool_idle(c);
+    free_b += c->cap_side + pool_idle(c, c->stream);
     if (free_b <= beside + kEscapeMargin &&
         free_b + (c->cap_main - mb) + (c->cap_blk - bb) > beside + kEscapeMargin) {
       cudaFree(c->d_main);
@@ -371,13 +390,13 @@ static fdp_status ensure_state(fdp_ctx *c, int W, int lanes, size_t beside) {
 // Residues a pass of fdp_run_sync really holds: `lanes`, or one span of 8 where the
 // fused row tail's escape words fit beside 8 lanes but not beside all of them
 // (n = 22, 14 lanes: 16.4 s in one pass of single cells, 13.5 s as passes of 8 and 6).
-static int lanes_with_escapes(const fdp_ctx *c, int W, int lanes) {
+static int lanes_with_escapes(fdp_ctx *c, int W, int lanes) {
   if (lanes <= 8 || !c->cfg.tail || whole_pass(c, W)) return lanes;
   const size_t state = size_t(fdp::main_states(W) + fdp::blocked_states(W)) * 4, esc = fdp::tail_escape_words(W) * 4;
   size_t free_b = 0, total_b = 0;
   if (!esc || (state + esc) * size_t(lanes) < (size_t(32) << 30) || cudaMemGetInfo(&free_b, &total_b) != cudaSuccess)
     return lanes;
-  const size_t have = free_b + pool_idle(c) + c->cap_side + c->cap_main + c->cap_blk;
+  const size_t have = free_b + pool_idle(c, c->stream) + c->cap_side + c->cap_main + c->cap_blk;
   return (state + esc) * size_t(lanes) + kEscapeMargin > have && (state + esc) * 8 + kEscapeMargin <= have ? 8 : lanes;
 }
 
@@ -586,7 +605,8 @@ extern "C" fdp_status fdp_run_sync(fdp_ctx *c, const fdp_problem *pr, uint32_t *
 // Escape words for one window of fdp_apply_cells, or null: allocated and freed
 // in the order of the caller's stream, so windows on other streams get words of
 // their own.  A pool that would have to grow leaves at least half of what is free
-// to others.  A window that needs more than the pool keeps (mapping fresh memory
+// to others, however many windows are in flight (at most kWindows; events say which
+// are).  A window that needs more than the pool keeps (mapping fresh memory
 // for each window costs more than the fused tail gives), or a stream under capture
 // (the captured work must not depend on an allocation of this context), runs cell
 // by cell.
@@ -598,8 +618,8 @@ static uint32_t *window_escapes(fdp_ctx *c, int W, int lanes, cudaStream_t st) {
     return nullptr;
   }
   void *p = nullptr;
-  bool ok = fdp::prepare_tail(W) == cudaSuccess;
-  const size_t idle = pool_idle(c);
+  const size_t idle = pool_idle(c, st);
+  bool ok = c->windows.size() < kWindows && fdp::prepare_tail(W) == cudaSuccess;
   if (ok && bytes > idle) {
     size_t free_b = 0, total_b = 0;
     ok = cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b / 2 > bytes - idle;
@@ -609,6 +629,16 @@ static uint32_t *window_escapes(fdp_ctx *c, int W, int lanes, cudaStream_t st) {
     return nullptr;
   }
   return static_cast<uint32_t *>(p);
+}
+
+// Gives a window's words back in the order of its stream.
+static cudaError_t window_done(fdp_ctx *c, int W, int lanes, uint32_t *esc, cudaStream_t st) {
+  cudaError_t e = cudaFreeAsync(esc, st);
+  WindowUse w{st, nullptr, size_t(fdp::tail_escape_words(W)) * lanes * 4};
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&w.done, cudaEventDisableTiming);
+  if (e != cudaSuccess) return e;
+  c->windows.push_back(w);
+  return cudaEventRecord(w.done, st);
 }
 
 extern "C" fdp_status fdp_apply_cells(fdp_ctx *c, int width, int p_hi, int p_lo, int lanes, const uint32_t *moduli,
@@ -643,7 +673,7 @@ extern "C" fdp_status fdp_apply_cells(fdp_ctx *c, int width, int p_hi, int p_lo,
   if (esc) {
     if (e == cudaSuccess) e = fdp::launch_tail(*t, lanes, moduli, d_main, d_block, esc, st, nullptr);
     if (e == cudaSuccess) e = cudaMemsetAsync(d_block, 0, size_t(fdp::blocked_states(width)) * lanes * 4, st);
-    const cudaError_t fe = cudaFreeAsync(esc, st);
+    const cudaError_t fe = window_done(c, width, lanes, esc, st);
     if (e == cudaSuccess) e = fe;
   }
   FDP_CK(e, "cell");

@@ -9,6 +9,14 @@
 #include "../../include/oneesan_fdp.h"
 #include "fdp_launch.h"
 
+// A window of fdp_apply_cells that took escape words: they are free for other
+// streams when `done` has been reached.
+struct WindowUse {
+  cudaStream_t stream;
+  cudaEvent_t done;
+  size_t bytes;
+};
+
 struct fdp_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -18,6 +26,7 @@ struct fdp_ctx {
   char *d_side = nullptr;                // what a synchronous call takes beside its state
   size_t cap_main = 0, cap_blk = 0, cap_side = 0;
   cudaMemPool_t pool = nullptr;          // escape words of fdp_apply_cells, stream-ordered
+  std::vector<WindowUse> windows;        // those whose pool memory may still be in use
   unsigned long long *d_acc = nullptr;   // first-row dot accumulators
   uint32_t *d_res = nullptr;             // residues on the device
   uint32_t *h_res = nullptr;             // residues, pinned host

@@ -98,3 +98,38 @@ def test_another_allocator_gets_what_a_window_left_in_the_pool():
         x = torch.empty(before - GIB // 2, dtype=torch.uint8, device="cuda")
         del x, a, b
         torch.cuda.empty_cache()
+
+
+def test_a_second_window_in_flight_leaves_half_of_what_is_free():
+    # Windows on two streams, the first held up by a delay: its words (910 MB at
+    # width 20, 4 lanes) are not idle although the call that frees them has returned,
+    # so the second window's may not be mapped beside them where less than twice as
+    # much is free; it runs cell by cell with the same result.
+    import torch
+    width, mods = 20, P[:4]
+    with fdp.Engine(0) as eng:
+        g = torch.Generator(device="cuda").manual_seed(1)
+        main = torch.randint(0, 2**31 - 1, (4 * orc.main_states(width),), dtype=torch.int32, device="cuda", generator=g)
+        blk = torch.randint(0, 2**31 - 1, (4 * orc.main_states(width - 1),), dtype=torch.int32, device="cuda", generator=g)
+        pairs = [(main.clone(), blk.clone()), (main, blk)]
+        streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+        small = [torch.zeros(n, dtype=torch.int32, device="cuda") for n in (4 * orc.main_states(14), 4 * orc.main_states(13))]
+        for s in streams:  # the library's tables and kernels
+            eng.apply_cells(14, 13, 1, mods, small[0].data_ptr(), small[1].data_ptr(), s.cuda_stream)
+        eng.apply_cells(width, 3, 2, mods, pairs[0][0].data_ptr(), pairs[0][1].data_ptr())
+        torch.cuda.synchronize()
+        pairs[0][0].copy_(main)
+        pairs[0][1].copy_(blk)
+        words = int(0.62 * 4 * 4 * orc.main_states(width))
+        fill = _fill(5 * words // 2)
+        before = torch.cuda.mem_get_info()[0]
+        with torch.cuda.stream(streams[0]):
+            torch.cuda._sleep(1_000_000_000)  # half a second
+        for s, (a, b) in zip(streams, pairs):
+            eng.apply_cells(width, width - 1, 1, mods, a.data_ptr(), b.data_ptr(), s.cuda_stream)
+        taken = before - torch.cuda.mem_get_info()[0]
+        torch.cuda.synchronize()
+        del fill
+        torch.cuda.empty_cache()
+        assert words // 2 < taken < 3 * words // 2
+        assert torch.equal(pairs[0][0], pairs[1][0]) and torch.equal(pairs[0][1], pairs[1][1])
