@@ -190,6 +190,7 @@ fdp_status fdp_ctx_tables_cap(fdp_ctx *c, int W, int cap, const DevTables **out)
   auto it = c->tables.find(key);
   if (it == c->tables.end()) {
     DevTables t;
+    const fdp::BesideCaptures beside;
     FDP_CK(fdp::upload_tables(W, cap, &t), "upload tables");
     it = c->tables.emplace(key, t).first;
   }
@@ -233,6 +234,7 @@ static bool whole_pass(const fdp_ctx *c, int W) {
 // Every device table a residue pass of width W reads, uploaded before any
 // stream capture starts (allocation and blocking copies cannot be captured).
 fdp_status fdp_prepare_pass(fdp_ctx *c, int W, const DevTables **full) {
+  const fdp::BesideCaptures beside;
   fdp_status s = fdp_ctx_tables(c, W, full);
   if (s != FDP_OK) return s;
   int rcap = 0;
@@ -257,6 +259,7 @@ fdp_status fdp_prepare_pass(fdp_ctx *c, int W, const DevTables **full) {
 // the windows in flight have handed their words back and without what the context
 // keeps for later calls.
 cudaError_t fdp_ctx_malloc(fdp_ctx *c, void **p, size_t bytes) {
+  const fdp::BesideCaptures beside;
   cudaError_t e = cudaMalloc(p, bytes);
   if (e != cudaErrorMemoryAllocation || (!c->pool && !c->d_side)) return e;
   cudaGetLastError();
@@ -328,6 +331,7 @@ struct SideMemory {
     if (c->cap_side > kSideKeep) drop();
   }
   void drop() {
+    const fdp::BesideCaptures beside;
     if (c->d_side) cudaFree(c->d_side);
     c->d_side = nullptr;
     c->cap_side = 0;
@@ -658,6 +662,7 @@ extern "C" fdp_status fdp_apply_cells(fdp_ctx *c, int width, int p_hi, int p_lo,
   for (int i = 0; i < lanes; ++i)
     if (moduli[i] < 2) return FDP_ERR_MODULUS;
   std::lock_guard<std::mutex> lk(c->mu);
+  const fdp::BesideCaptures beside;  // a kernel's first launch loads it, too
   FDP_CK(cudaSetDevice(c->device), "cudaSetDevice");
   const DevTables *t = nullptr;
   fdp_status s = fdp_ctx_tables(c, width, &t);

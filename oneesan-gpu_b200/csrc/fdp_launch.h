@@ -84,6 +84,18 @@ cudaError_t launch_ternary_index_chunked(int chunk, const uint32_t *codes, uint3
 
 int device_sm_count();
 
+// While it lives, this thread's allocations, blocking copies, event queries and
+// loads of kernels do not invalidate a capture that runs on another stream (of any
+// thread, in any mode): what a call sets up on first use must not depend on who
+// captures meanwhile.
+struct BesideCaptures {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  BesideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~BesideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  BesideCaptures(const BesideCaptures &) = delete;
+  BesideCaptures &operator=(const BesideCaptures &) = delete;
+};
+
 #if defined(__CUDACC__)
 // Small launches of one chain overlap at their seams: a kernel launched with
 // `overlap` starts once the CTAs of the one before it have all started, if there

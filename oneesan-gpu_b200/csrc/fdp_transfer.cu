@@ -619,6 +619,7 @@ extern "C" fdp_status fdp_reverse2_apply(fdp_ctx *c, int width, int p, int lanes
   }
   fdp_status s = check_apply(width, lanes, moduli, d_in_main, d_in_block, d_out_main, d_out_block);
   if (s != FDP_OK) return s;
+  const fdp::BesideCaptures beside;
   cudaError_t e = cudaSetDevice(c->device);
   if (e != cudaSuccess) return fdp_cuda_status(e, "cudaSetDevice");
   const Counts *cnt = device_counts();
@@ -627,9 +628,9 @@ extern "C" fdp_status fdp_reverse2_apply(fdp_ctx *c, int width, int p, int lanes
   launch_apply(c, width, lanes, moduli, d_in_main, d_in_block, d_out_main, d_out_block, stream, &a);
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : c->stream;
   // The inputs, reduced, go to the outputs, and the two cells run there in place:
-  // no ranks of sources, whole panel words.  Unaligned pointers, tiny vectors and
-  // streams under capture (the width's tables may have to be uploaded) enumerate
-  // the sources of the sources.  The line: three launches take 20 us, the
+  // no ranks of sources, whole panel words.  Unaligned pointers, tiny vectors,
+  // streams under capture (the width's tables may have to be uploaded) and widths
+  // whose tables find no memory enumerate the sources of the sources.  The line: three launches take 20 us, the
   // enumeration 23 us for one lane of width 8 (708 words), 816 against 41 us for
   // 8 lanes of width 15.
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -638,13 +639,16 @@ extern "C" fdp_status fdp_reverse2_apply(fdp_ctx *c, int width, int p, int lanes
   if (aligned && (a.M + a.D) * ull(lanes) >= kReverse2InPlace &&
       cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
     const fdp::DevTables *t = nullptr;
-    if ((s = fdp_ctx_tables(c, width, &t)) != FDP_OK) return s;
-    const int panels = lanes / 8 + __builtin_popcount(unsigned(lanes % 8));
-    copy_residues_kernel<<<dim3(grid_for(a.M + a.D), unsigned(panels)), 256, 0, st>>>(a);
-    e = cudaGetLastError();
-    for (int q = p; q >= p - 1 && e == cudaSuccess; --q)
-      e = fdp::launch_cell(*t, lanes, moduli, d_out_main, d_out_block, q, false, true, fdp::LaunchCfg{}, st);
-    return fdp_cuda_status(e, "reverse2");
+    s = fdp_ctx_tables(c, width, &t);
+    if (s != FDP_OK && s != FDP_ERR_HBM) return s;
+    if (t) {
+      const int panels = lanes / 8 + __builtin_popcount(unsigned(lanes % 8));
+      copy_residues_kernel<<<dim3(grid_for(a.M + a.D), unsigned(panels)), 256, 0, st>>>(a);
+      e = cudaGetLastError();
+      for (int q = p; q >= p - 1 && e == cudaSuccess; --q)
+        e = fdp::launch_cell(*t, lanes, moduli, d_out_main, d_out_block, q, false, true, fdp::LaunchCfg{}, st);
+      return fdp_cuda_status(e, "reverse2");
+    }
   }
   reverse2_kernel<<<grid_for(a.M + a.D), 256, 0, st>>>(a, cnt, width, p);
   return fdp_cuda_status(cudaGetLastError(), "reverse2");

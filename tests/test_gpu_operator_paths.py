@@ -65,3 +65,36 @@ def test_reverse2_under_capture(engine):
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(c, e) and torch.equal(d, f)
+
+
+def test_first_calls_of_a_width_beside_another_streams_capture():
+    # What these calls set up on first use (tables, the windows' pool) leaves a
+    # capture that runs on another stream alone, also where that is refused to
+    # the thread ("global").
+    import torch
+    with fdp.Engine(0) as eng:
+        x = torch.zeros(1024, dtype=torch.int32, device="cuda")
+        other = torch.cuda.Stream()
+        a, b, c, d = _vectors(13, 1, 0, 5)
+        r2 = _vectors(15, 1, 0, 6)[:2]
+        r2 = [torch.remainder(t.to(torch.int64), 97).to(torch.int32) for t in r2]
+        again = [t.clone() for t in r2]
+        mods, wmods = [4294967291], [97]
+        w = _vectors(12, 1, 0, 7)
+        eng.reverse2_apply(12, 5, mods, *[t.data_ptr() for t in w])  # the library's kernels and count table
+        graph = torch.cuda.CUDAGraph()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph, capture_error_mode="global"):
+            x += 1
+            eng.reverse2_apply(13, 5, mods, a.data_ptr(), b.data_ptr(), c.data_ptr(), d.data_ptr(), other.cuda_stream)
+            eng.apply_cells(15, 14, 1, wmods, r2[0].data_ptr(), r2[1].data_ptr(), other.cuda_stream)
+            x += 1
+        graph.replay()
+        torch.cuda.synchronize()
+        assert int(x[0]) == 2
+        got = c.clone(), d.clone()
+        eng.reverse2_apply(13, 5, mods, a.data_ptr(), b.data_ptr(), c.data_ptr(), d.data_ptr())
+        eng.apply_cells(15, 14, 1, wmods, again[0].data_ptr(), again[1].data_ptr())
+        torch.cuda.synchronize()
+        assert torch.equal(got[0], c) and torch.equal(got[1], d)
+        assert torch.equal(r2[0], again[0]) and torch.equal(r2[1], again[1])
