@@ -286,10 +286,12 @@ fdp_status fdp_server_get_stats(fdp_ctx *ctx, fdp_server_stats *stats);
  * kernel's scheduling knobs one at a time (lane_items, share_min,
  * compact_max_p, compact_carry, compact_items, and split_spans_min_p above 8 lanes; a change
  * is kept when the row is at least 0.5 % faster).  Each sample is a timed row sweep of the problem's own n on
- * the context's state buffers; the score is the estimated device seconds per
- * residue.  The known-answer check runs the tuned configuration at the
- * problem's own n when the reference publishes a residue mod 4294967291 for
- * it (n = 9, 18, 20, 21, 22, 23), else at n = 9.  The winner is applied to the context
+ * the context's state buffers, as a pass runs it (low cells fused where memory
+ * allows; a residue count that no pass would hold is listed and not timed); the
+ * score is the estimated device seconds per residue.  The known-answer check
+ * runs the tuned configuration at the problem's own n when the reference
+ * publishes a residue mod 4294967291 for it (n = 9, 18, 20, 21, 22, 23), else at
+ * n = 9, there cell by cell.  The winner is applied to the context
  * (fdp_set_tuning) and returned; json_out (if not NULL) receives every
  * candidate record as a JSON document of at most json_cap bytes.
  */

@@ -432,6 +432,48 @@ extern "C" fdp_status fdp_test_inject_pass_errors(int count) {
   return FDP_OK;
 }
 
+// `rows` row sweeps in the full space: each row's cells one launch each, or, given
+// escape words, cells s-1..1 of it as one fused pass.
+static fdp_status enqueue_full_rows(fdp_ctx *c, const DevTables &t, int L, const uint32_t *mods, uint32_t *main,
+                                    uint32_t *blk, uint32_t *esc, int rows, cudaStream_t s, uint64_t *n,
+                                    cudaStream_t span_stream, cudaEvent_t fork, cudaEvent_t join) {
+  const int W = t.W;
+  const bool fused = esc && c->cfg.tail && fdp::tail_symbols(W);
+  auto cells = [&](int lanes, const uint32_t *m, uint32_t *mn, uint32_t *bk, int last, cudaStream_t ss) {
+    cudaError_t e = cudaSuccess;
+    for (int p = W - 1; p >= last && e == cudaSuccess; --p)
+      e = fdp::launch_cell(t, lanes, m, mn, bk, p, p == W - 1, false, c->cfg, ss, n);
+    return e;
+  };
+  // Span chains overlap the tails of single-cell launches; with the fused row
+  // tail one chain is faster (n = 20, 14 lanes: 1.40 against 1.53 s), as its CTAs
+  // take whole SMs and hold back the other chain's.
+  if (!fused && span_stream && fork && join && c->cfg.span_chains && L > 8 && !c->cfg.split_panels &&
+      c->cfg.split_spans_min_p <= 1 && rows > 0) {
+    // Each lane span is laid out as a lane count of its own at its first
+    // panel's offset and no cell reads another span's panels, so the spans'
+    // row sweeps run as two chains of launches, joined before the read-out.
+    FDP_CK(cudaEventRecord(fork, s), "span fork");
+    FDP_CK(cudaStreamWaitEvent(span_stream, fork, 0), "span fork");
+    for (int l0 = 0, i = 0; l0 < L; ++i) {
+      const int le = fdp::span_end_of(L, l0);
+      for (int row = 0; row < rows; ++row)
+        FDP_CK(cells(le - l0, mods + l0, main + size_t(l0) * fdp::main_states(W),
+                     blk + size_t(l0) * fdp::blocked_states(W), 1, i == 0 ? s : span_stream),
+               "cell");
+      l0 = le;
+    }
+    FDP_CK(cudaEventRecord(join, span_stream), "span join");
+    FDP_CK(cudaStreamWaitEvent(s, join, 0), "span join");
+    return FDP_OK;
+  }
+  for (int row = 0; row < rows; ++row) {
+    FDP_CK(cells(L, mods, main, blk, fused ? fdp::tail_symbols(W) : 1, s), "cell");
+    if (fused) FDP_CK(fdp::launch_tail(t, L, mods, main, blk, esc, s, n), "row tail");
+  }
+  return FDP_OK;
+}
+
 fdp_status fdp_enqueue_pass(fdp_ctx *c, const DevTables &t, int L, const uint32_t *mods, uint32_t *main,
                             uint32_t *blk, uint32_t *esc, unsigned long long *acc, uint32_t *d_res, uint32_t *h_res,
                             unsigned int *d_err, cudaStream_t s, uint64_t *launches, cudaStream_t span_stream,
@@ -490,43 +532,9 @@ fdp_status fdp_enqueue_pass(fdp_ctx *c, const DevTables &t, int L, const uint32_
   }
   if (prev != &t) FDP_CK(fdp::enqueue_expand(*prev, t, L, main, blk, D * uint64_t(L), s, &n), "grow state");
   const int row0 = next_row > B + 1 ? next_row : B + 1;
-  const bool fused = esc && c->cfg.tail && fdp::tail_symbols(W);
-  // One row in the full space: its cells one launch each, or, given escape
-  // words, cells s-1..1 as one fused pass.
-  auto full_row = [&](int lanes, const uint32_t *m, uint32_t *mn, uint32_t *bk, uint32_t *es,
-                      cudaStream_t ss) -> fdp_status {
-    const int last = fused ? fdp::tail_symbols(W) : 1;
-    for (int p = W - 1; p >= last; --p)
-      FDP_CK(fdp::launch_cell(t, lanes, m, mn, bk, p, p == W - 1, false, c->cfg, ss, &n), "cell");
-    if (last > 1) FDP_CK(fdp::launch_tail(t, lanes, m, mn, bk, es, ss, &n), "row tail");
-    return FDP_OK;
-  };
-  // Span chains overlap the tails of single-cell launches; with the fused row
-  // tail one chain is faster (n = 20, 14 lanes: 1.40 against 1.53 s), as its CTAs
-  // take whole SMs and hold back the other chain's.
-  const bool chains = !fused && span_stream && fork && join && c->cfg.span_chains && L > 8 && !c->cfg.split_panels &&
-                      c->cfg.split_spans_min_p <= 1 && row0 <= fdp::sweep_rows(W);
-  if (chains) {
-    // Each lane span is laid out as a lane count of its own at its first
-    // panel's offset and no cell reads another span's panels, so the spans'
-    // row sweeps run as two chains of launches, joined before the read-out.
-    FDP_CK(cudaEventRecord(fork, s), "span fork");
-    FDP_CK(cudaStreamWaitEvent(span_stream, fork, 0), "span fork");
-    for (int l0 = 0, i = 0; l0 < L; ++i) {
-      const int le = fdp::span_end_of(L, l0);
-      cudaStream_t ss = i == 0 ? s : span_stream;
-      for (int row = row0; row <= fdp::sweep_rows(W); ++row)
-        if ((st = full_row(le - l0, mods + l0, main + size_t(l0) * M, blk + size_t(l0) * D,
-                           esc ? esc + size_t(l0) * fdp::tail_escape_words(W) : nullptr, ss)) != FDP_OK)
-          return st;
-      l0 = le;
-    }
-    FDP_CK(cudaEventRecord(join, span_stream), "span join");
-    FDP_CK(cudaStreamWaitEvent(s, join, 0), "span join");
-  } else {
-    for (int row = row0; row <= fdp::sweep_rows(W); ++row)
-      if ((st = full_row(L, mods, main, blk, esc, s)) != FDP_OK) return st;
-  }
+  if ((st = enqueue_full_rows(c, t, L, mods, main, blk, esc, fdp::sweep_rows(W) - row0 + 1, s, &n, span_stream, fork,
+                              join)) != FDP_OK)
+    return st;
   FDP_CK(fdp::launch_first_row_dot(t, L, mods, main, acc, d_res, s), "first-row dot");
   n += 2;
   if (h_res) FDP_CK(cudaMemcpyAsync(h_res, d_res, sizeof(uint32_t) * L, cudaMemcpyDeviceToHost, s), "residue copy");
@@ -603,6 +611,65 @@ extern "C" fdp_status fdp_run_sync(fdp_ctx *c, const fdp_problem *pr, uint32_t *
   acc.transitions = po.transitions_per_residue * uint64_t(pr->k);
   acc.wall_s = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
   if (st) *st = acc;
+  return FDP_OK;
+}
+
+int fdp_pass_lanes(fdp_ctx *c, int n, int lanes) {
+  std::lock_guard<std::mutex> lk(c->mu);
+  return cudaSetDevice(c->device) == cudaSuccess ? lanes_with_escapes(c, n + 1, lanes) : lanes;
+}
+
+bool fdp_pass_is_whole(fdp_ctx *c, int n) {
+  std::lock_guard<std::mutex> lk(c->mu);
+  return whole_pass(c, n + 1);
+}
+
+void fdp_pass_single_cells(fdp_ctx *c, bool on) {
+  std::lock_guard<std::mutex> lk(c->mu);
+  c->cfg.tail = !on;
+}
+
+fdp_status fdp_time_pass_row(fdp_ctx *c, const fdp_problem *pr, double *row_ms) {
+  fdp_status s = check_problem(pr);
+  if (s != FDP_OK) return s;
+  std::lock_guard<std::mutex> lk(c->mu);
+  FDP_CK(cudaSetDevice(c->device), "cudaSetDevice");
+  const int W = pr->n + 1, L = pr->lanes < pr->k ? pr->lanes : pr->k;
+  if (W < 3) return FDP_ERR_ARGS;
+  const DevTables *t = nullptr;
+  if ((s = fdp_prepare_pass(c, W, &t)) != FDP_OK) return s;
+  const bool whole = whole_pass(c, W);
+  SideMemory esc(c);
+  if (!whole) {
+    const size_t eb = c->cfg.tail ? size_t(fdp::tail_escape_words(W)) * L * 4 : 0;
+    if ((s = ensure_state(c, W, L, eb)) != FDP_OK) return s;
+    if (eb) esc.take_optional(eb, kEscapeMargin);
+  }
+  const int rows = whole ? fdp::sweep_rows(W) : (W < 19 ? 8 : 1);  // some ms together
+  cudaGraph_t g = nullptr;
+  cudaGraphExec_t ge = nullptr;
+  uint64_t n = 0;
+  FDP_CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
+  fdp_status es = whole ? cuda_status(fdp::launch_whole(W, L, pr->moduli, c->d_res, c->stream), "whole solve")
+                        : enqueue_full_rows(c, *t, L, pr->moduli, c->d_main, c->d_blk,
+                                            reinterpret_cast<uint32_t *>(esc.p), rows, c->stream, &n, c->span_stream,
+                                            c->span_fork, c->span_join);
+  cudaError_t e = cudaStreamEndCapture(c->stream, &g);
+  if (es == FDP_OK) es = cuda_status(e, "end capture");
+  if (es == FDP_OK) es = cuda_status(cudaGraphInstantiate(&ge, g, 0), "graph instantiate");
+  if (g) cudaGraphDestroy(g);
+  for (int i = 0; i < 2 && es == FDP_OK; ++i) {  // the first one untimed
+    cudaEventRecord(c->ev0, c->stream);
+    es = cuda_status(cudaGraphLaunch(ge, c->stream), "graph launch");
+    cudaEventRecord(c->ev1, c->stream);
+    const cudaError_t se = cudaStreamSynchronize(c->stream);
+    if (es == FDP_OK) es = cuda_status(se, "timed rows");
+  }
+  if (ge) cudaGraphExecDestroy(ge);
+  if (es != FDP_OK) return es;
+  float ms = 0;
+  cudaEventElapsedTime(&ms, c->ev0, c->ev1);
+  *row_ms = double(ms) / rows;
   return FDP_OK;
 }
 

@@ -62,6 +62,16 @@ fdp_status fdp_enqueue_pass(fdp_ctx *c, const fdp::DevTables &t, int L, const ui
                             unsigned int *d_err, cudaStream_t s, uint64_t *launches,
                             cudaStream_t span_stream = nullptr, cudaEvent_t fork = nullptr,
                             cudaEvent_t join = nullptr);
+// Residues a pass of fdp_run_sync holds when `lanes` are asked for.
+int fdp_pass_lanes(fdp_ctx *c, int n, int lanes);
+// Whether its pass is one launch, which reads no tuning of the cell kernels.
+bool fdp_pass_is_whole(fdp_ctx *c, int n);
+// Every cell its own launch, whatever the width and the memory.
+void fdp_pass_single_cells(fdp_ctx *c, bool on);
+// Time of a row of one pass of pr->lanes residues as fdp_run_sync runs it: from a
+// graph, the low cells fused where that pass would fuse them, after an untimed run.
+// A pass of one launch counts as sweep_rows rows.
+fdp_status fdp_time_pass_row(fdp_ctx *c, const fdp_problem *pr, double *row_ms);
 // A computation's error word: a kernel that gives up on a bounded wait writes
 // a nonzero value to it.  Each computation (a run_sync graph, one problem of a
 // run_multi_sync graph, one served request) owns its word in its own buffers;

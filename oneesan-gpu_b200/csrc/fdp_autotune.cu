@@ -2,10 +2,15 @@
 // (1 warm-up + `repeats`, median), estimated device seconds per residue, and a
 // known-residue check of the winner at the problem's own n when the reference
 // publishes a residue mod 4294967291 for it (else n = 9, 2674633373,
-// scripts/test/groupbatch-runtime.py:17).
+// scripts/test/groupbatch-runtime.py:17; its passes are one launch that reads no
+// tuning, so the check runs them cell by cell).  A row is timed as a pass runs it
+// (fdp_time_pass_row): with the low cells fused where memory allows, and with the
+// residues such a pass really holds; a last pass of fewer residues counts with its
+// own time.
 //
 // Stage 1 searches how the k moduli split into passes (lanes), one launch vs
-// one launch per lane panel, and the CTA size.  Stage 2 then tunes the cell
+// one launch per lane panel, and the CTA size.  Stage 2 (not where a pass is one
+// launch) then tunes the cell
 // kernel's scheduling knobs of the winner one at a time (coordinate descent,
 // a change kept only when the row is at least 0.5 % faster): the warp chunk
 // (lane_items), the shortest shared prefix decode (share_min), the highest
@@ -80,7 +85,28 @@ extern "C" fdp_status fdp_autotune(fdp_ctx *c, const fdp_problem *pr, uint64_t b
   fdp_autotune_result best{};
   best.s_per_residue = INFINITY;
   int tried = 0, rejected = 0;
-  std::vector<double> cell_ms(size_t(W) + 1);
+  // Time of one row in every pass of the k moduli at L residues a pass (`all`), and
+  // in the first of them (`row`): medians of `repeats`, after one not counted.
+  auto sample = [&](int L, double *row, double *all) -> fdp_status {
+    const int last = k - (k - 1) / L * L;
+    const fdp_problem full{pr->n, L, pr->moduli, L}, rest{pr->n, last, pr->moduli, last};
+    std::vector<double> rows_ms, alls;
+    for (int r = 0; r <= repeats; ++r) {
+      double a = 0, b = 0;
+      fdp_status s = fdp_time_pass_row(c, &full, &a);
+      b = a;
+      if (s == FDP_OK && last != L) s = fdp_time_pass_row(c, &rest, &b);
+      if (s != FDP_OK) return s;
+      if (r > 0) {
+        rows_ms.push_back(a);
+        alls.push_back(a * ((k - 1) / L) + b);
+      }
+    }
+    *row = median(rows_ms);
+    *all = median(alls);
+    return FDP_OK;
+  };
+  double best_all = 0;
   for (int L : lane_opts) {
     fdp_problem cand{pr->n, L, pr->moduli, L};
     fdp_plan_out plan{};
@@ -93,6 +119,12 @@ extern "C" fdp_status fdp_autotune(fdp_ctx *c, const fdp_problem *pr, uint64_t b
       first = false;
       continue;
     }
+    if (const int held = fdp_pass_lanes(c, pr->n, L); held != L) {  // a candidate of its own
+      js += std::string(first ? "" : ",") + "{\"lanes\":" + std::to_string(L) + ",\"status\":\"runs as " +
+            std::to_string(held) + "\"}";
+      first = false;
+      continue;
+    }
     const int npanels = panel_count(L);
     for (int split = 0; split <= (npanels > 1 ? 1 : 0); ++split)
       for (int block : {128, 256}) {
@@ -101,13 +133,8 @@ extern "C" fdp_status fdp_autotune(fdp_ctx *c, const fdp_problem *pr, uint64_t b
         t.grid = 0;
         t.split_panels = split;
         fdp_status s = fdp_set_tuning(c, &t);
-        std::vector<double> samples;
-        for (int r = 0; r <= repeats && s == FDP_OK; ++r) {
-          s = fdp_time_cells(c, &cand, 1, cell_ms.data());
-          double row = 0;
-          for (int p = 1; p < W; ++p) row += cell_ms[size_t(p)];
-          if (r > 0) samples.push_back(row);
-        }
+        double row = 0, all = 0;
+        if (s == FDP_OK) s = sample(L, &row, &all);
         ++tried;
         char buf[320];
         if (s != FDP_OK) {
@@ -119,12 +146,11 @@ extern "C" fdp_status fdp_autotune(fdp_ctx *c, const fdp_problem *pr, uint64_t b
           fdp_set_tuning(c, &saved);
           return s;
         }
-        const double row = median(samples);
         const int passes = (k + L - 1) / L;
         // Each pass sweeps the rows the row-k initialiser does not fill
         // (its own fill is left out of the estimate); spread over k residues.
         const int swept = rows - (plan.init_rows >= 2 ? plan.init_rows - 1 : 0);
-        const double spr = row * 1e-3 * swept * passes / k;
+        const double spr = all * 1e-3 * swept / k;
         snprintf(buf, sizeof(buf),
                  "%s{\"lanes\":%d,\"split_panels\":%d,\"block\":%d,\"status\":\"ok\",\"row_ms\":%.4f,"
                  "\"s_per_residue\":%.6f,\"passes\":%d}",
@@ -137,6 +163,7 @@ extern "C" fdp_status fdp_autotune(fdp_ctx *c, const fdp_problem *pr, uint64_t b
           best.tuning = t;
           best.row_ms = row;
           best.s_per_residue = spr;
+          best_all = all;
         }
       }
   }
@@ -158,11 +185,10 @@ extern "C" fdp_status fdp_autotune(fdp_ctx *c, const fdp_problem *pr, uint64_t b
                         {"compact_carry", &fdp_tuning::compact_carry, {-1, 1}},
                         {"compact_items", &fdp_tuning::compact_items, {1, 2, 4, 8}},
                         {"split_spans_min_p", &fdp_tuning::split_spans_min_p, {1, 8, 1000}}};
-  {
+  if (!fdp_pass_is_whole(c, pr->n)) {
     fdp_problem cand{pr->n, best.lanes, pr->moduli, best.lanes};
     fdp_tuning cur{};
     fdp_get_tuning(c, &cur);  // the winner with its defaults resolved
-    const int passes = (k + best.lanes - 1) / best.lanes;
     fdp_plan_out plan{};
     fdp_plan(&cand, budget, &plan);
     const int swept = rows - (plan.init_rows >= 2 ? plan.init_rows - 1 : 0);
@@ -175,23 +201,17 @@ extern "C" fdp_status fdp_autotune(fdp_ctx *c, const fdp_problem *pr, uint64_t b
         fdp_tuning t = cur;
         t.*kb.field = v;
         if (fdp_set_tuning(c, &t) != FDP_OK) continue;
-        std::vector<double> samples;
-        for (int r = 0; r <= repeats && s == FDP_OK; ++r) {
-          s = fdp_time_cells(c, &cand, 1, cell_ms.data());
-          double row = 0;
-          for (int p = 1; p < W; ++p) row += cell_ms[size_t(p)];
-          if (r > 0) samples.push_back(row);
-        }
-        if (s != FDP_OK) break;
+        double row = 0, all = 0;
+        if ((s = sample(best.lanes, &row, &all)) != FDP_OK) break;
         ++tried;
-        const double row = median(samples);
-        const double spr = row * 1e-3 * swept * passes / k;
+        const double spr = all * 1e-3 * swept / k;
         char buf[320];
         snprintf(buf, sizeof(buf), ",{\"lanes\":%d,\"%s\":%d,\"status\":\"ok\",\"row_ms\":%.4f,\"s_per_residue\":%.6f}",
                  best.lanes, kb.name, v, row, spr);
         js += buf;
-        if (row < best.row_ms * 0.995) {
+        if (all < best_all * 0.995) {
           best.tuning = t;
+          best_all = all;
           best.row_ms = row;
           best.s_per_residue = spr;
           cur = t;
@@ -210,7 +230,10 @@ extern "C" fdp_status fdp_autotune(fdp_ctx *c, const fdp_problem *pr, uint64_t b
     std::vector<uint32_t> mods(size_t(best.lanes), m), res(size_t(best.lanes));
     fdp_problem chk{chk_known.n, best.lanes, mods.data(), best.lanes};
     fdp_run_stats st{};
+    const bool cells = fdp_pass_is_whole(c, chk_known.n);
+    if (cells) fdp_pass_single_cells(c, true);
     s = fdp_run_sync(c, &chk, res.data(), &st);
+    if (cells) fdp_pass_single_cells(c, false);
     if (s == FDP_OK)
       for (uint32_t r : res)
         if (r != chk_known.residue) {
