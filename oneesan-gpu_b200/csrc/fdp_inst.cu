@@ -34,7 +34,8 @@ cudaError_t launch_cell_t(const CellArgs &a, const LaunchCfg &cfg, cudaStream_t 
   if (cfg.block < 32 || cfg.block > 256 || cfg.block % 32) return cudaErrorInvalidValue;
   if (a.W < 2 || a.W > FDP_MAXW) return cudaErrorInvalidValue;
   const int compact = a.compact == 2 ? 2 : (a.compact && a.lane_items <= FDP_REC_MAX_ITEMS ? 1 : 0);
-  const bool runs = K <= 8 && a.runs != 0 && !a.compact && a.p >= 2;
+  constexpr bool kRuns = runs_range(sizeof(Idx) == 8, K).below > 0;
+  const bool runs = kRuns && a.runs != 0 && !a.compact && a.p >= 2;
   const size_t smem = cell_smem_bytes<Idx, K>(cfg.block, a.W, compact, a.lane_items);
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -54,7 +55,7 @@ cudaError_t launch_cell_t(const CellArgs &a, const LaunchCfg &cfg, cudaStream_t 
       if (e != cudaSuccess) return e;
       v.limit_set = true;
     }
-    if constexpr (K <= 8) {
+    if constexpr (kRuns) {
       if (runs && !v.runs_set) {
         e = cudaFuncSetAttribute(cell_run_kernel<Idx, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(CellSmem<Idx>)));
         if (e != cudaSuccess) return e;
@@ -63,7 +64,7 @@ cudaError_t launch_cell_t(const CellArgs &a, const LaunchCfg &cfg, cudaStream_t 
     }
     int &slot = v.per_sm[(uint64_t(runs ? 2 : (a.compact ? 1 : 0)) << 61) | (uint64_t(cfg.block) << 32) | uint64_t(smem)];
     if (slot == 0) {
-      if constexpr (K <= 8) {
+      if constexpr (kRuns) {
         if (runs) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&slot, cell_run_kernel<Idx, K>, cfg.block, smem);
       }
       if (!runs)
@@ -82,7 +83,7 @@ cudaError_t launch_cell_t(const CellArgs &a, const LaunchCfg &cfg, cudaStream_t 
   const uint64_t need = (a.items + per_block - 1) / per_block;
   if (uint64_t(grid) > need) grid = int(need ? need : 1);
   const bool overlap = 4 * grid <= 3 * device_sm_count() * per_sm;
-  if constexpr (K <= 8) {
+  if constexpr (kRuns) {
     if (runs) return launch_chained(cell_run_kernel<Idx, K>, unsigned(grid), unsigned(cfg.block), smem, s, a, overlap);
   }
   return a.compact ? launch_chained(cell_kernel<Idx, K>, unsigned(grid), unsigned(cfg.block), smem, s, a, overlap)

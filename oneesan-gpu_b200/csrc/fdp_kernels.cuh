@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(256, stream_min_blocks<K>()) cell_stream_kerne
   cell_body<Idx, K, false>(a);
 }
 
-// The streaming cells of lane counts up to 8, p >= 2, run by run.  Bound at one
+// The streaming cells, p >= 2, run by run, where runs_range says so.  Bound at one
 // lane: instruction issue (half the slots busy, of which the chunk's prefix walk
 // and closure scan take most, n = 20: 147 a warp of items, DRAM 2.9 TB/s); at 8
 // lanes: HBM.  Three CTAs per SM: 64 registers spill at most lane counts.

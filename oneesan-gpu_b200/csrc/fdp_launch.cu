@@ -88,14 +88,10 @@ static CellArgs schedule_cell(const CellArgs &in, int K, bool u64, const LaunchC
     a.lane_items = cfg.compact_items > 0 ? cfg.compact_items : kCarryItems;
     if (uint64_t(a.lane_items) > fill) a.lane_items = int(fill);
   }
-  // Streaming cells run by run where that is faster (a whole row's cells p >= 8).
-  // 32-bit ranks, n = 20: 1 lane 13.0 -> 11.4 ms, 6 lanes 32.5 -> 31.9, 8 lanes
-  // 39.7 -> 39.4, but 2 lanes 15.4 -> 16.9 and 4 lanes 22.2 -> 25.0 (the item
-  // kernel's 6 CTAs per SM hide more).  64-bit ranks, n = 23, where a decode
-  // costs twice the instructions: 1 lane 421 -> 262 ms, 2 lanes 464 -> 419, 5
-  // lanes 771 -> 737, but 4 lanes 618 -> 632; their chunks are four times as long
-  // (1 lane 308 -> 262 ms; at n = 20 longer chunks are slower, 11.4 -> 12.6 ms).
-  a.runs = !a.compact && (K == 1 || (K >= 6 && K <= 8) || (u64 && (K == 2 || K == 5))) ? 1 : 0;
+  const RunsRange r = runs_range(u64, K);
+  a.runs = !a.compact && fill >= r.from && fill < r.below ? 1 : 0;
+  // At 64 bits a run kernel's chunks are four times as long (n = 23, one lane: 308
+  // -> 262 ms; at 32 bits longer chunks are slower, n = 20 11.4 -> 12.6 ms).
   if (a.runs && u64 && uint64_t(a.lane_items) * 4 <= fill) a.lane_items *= 4;
   return a;
 }

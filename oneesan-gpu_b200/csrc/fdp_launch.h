@@ -14,6 +14,39 @@ constexpr int kMaxLanes = 16;  // K = 1..16 residues interleaved per state
 constexpr int kCarryItems = 16;  // default states per lane of a grouped chunk with carry-over queues
 
 // Per-(width, height cap) device table blob.
+// Where the streaming cells of a span of K lanes go run by run (cell_run_kernel)
+// instead of item by item: from `from` to below `below` items per resident thread.
+// A run shares one decode and one closure scan among its items, but three CTAs per
+// SM hold less in flight than the item kernel's four to six, and a chunk of one or
+// two items a lane has nothing to share.  Cells p >= 9 of a row, item by item and
+// run by run, in ms:
+//   lanes      n = 14        16          18          20           22
+//   1       0.071 0.090  0.320 0.339  1.82 1.62  11.7 10.1   99.3  83.2
+//   2       0.074 0.090  0.336 0.389  2.14 2.30  14.0 15.3  118   127
+//   3       0.086 0.089  0.492 0.434  3.35 2.91  21.4 21.2  177   184
+//   4       0.077 0.087  0.456 0.515  2.81 3.12  20.4 22.8  178   196
+//   5       0.091 0.090  0.735 0.592  3.90 3.38  29.8 25.8  262   228
+//   6       0.091 0.092  0.738 0.658  3.89 3.71  29.8 29.1  270   264
+//   7       0.095 0.100  0.815 0.831  4.47 4.75  35.7 36.2  329   324
+//   8       0.094 0.096  0.803 0.786  4.53 4.58  36.6 36.2  331   326
+// 64-bit ranks (n = 23), where a decode costs twice the instructions: 1 lane 385
+// 238, 2 428 390, 3 585 553, 4 572 590, 5 714 684; six lanes do not fit a device.
+struct RunsRange {
+  uint64_t from, below;
+};
+constexpr RunsRange runs_range(bool u64, int K) {
+  constexpr uint64_t all = ~uint64_t(0);
+  if (u64) return K == 1 || K == 2 || K == 3 || K == 5 ? RunsRange{0, all} : RunsRange{0, 0};
+  switch (K) {
+    case 1: return {16, all};   // n >= 17 (0.682 0.622 there)
+    case 3: return {0, 1024};   // n <= 20 (n = 21 59.8 61.4)
+    case 5:
+    case 6: return {0, all};
+    case 8: return {8, all};    // n >= 16 (n = 15 0.196 0.204)
+    default: return {0, 0};
+  }
+}
+
 struct DevTables {
   void *ptr = nullptr;
   bool u64 = false;
