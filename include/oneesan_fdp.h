@@ -407,6 +407,16 @@ fdp_status fdp_first_row_dot_noalloc(int width, int lanes, const uint32_t *modul
  */
 fdp_status fdp_test_inject_pass_errors(int count);
 
+/*
+ * Tests of the passes that memory or size decide on.  fdp_test_single_cells: with
+ * `on`, every pass and window of the context runs each cell as its own launch, as
+ * where no memory is left for the fused low cells.  fdp_test_pass_lanes: residues a
+ * pass of fdp_run_sync holds at grid size n when `lanes` are asked for and
+ * have_bytes of device memory serve its state and workspace (no device access).
+ */
+fdp_status fdp_test_single_cells(fdp_ctx *ctx, int on);
+int fdp_test_pass_lanes(int n, int lanes, uint64_t have_bytes);
+
 /* Canonical rank / unrank of frontier words on the device (GB.cu:1568 rank_full). */
 fdp_status fdp_rank_words(fdp_ctx *ctx, int width, const uint64_t *d_words, uint64_t *d_ranks, uint64_t count,
                           void *stream);

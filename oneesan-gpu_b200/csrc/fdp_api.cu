@@ -391,17 +391,38 @@ static fdp_status ensure_state(fdp_ctx *c, int W, int lanes, size_t beside) {
   return s;
 }
 
-// Residues a pass of fdp_run_sync really holds: `lanes`, or one span of 8 where the
-// fused row tail's escape words fit beside 8 lanes but not beside all of them
-// (n = 22, 14 lanes: 16.4 s in one pass of single cells, 13.5 s as passes of 8 and 6).
+// Whether passes of more than 8 lanes are large enough (32 GiB with the fused row
+// tail's escape words) to be split where memory asks for it.
+static bool may_split(int W, int lanes) {
+  const uint64_t esc = fdp::tail_escape_words(W), lane = fdp::main_states(W) + fdp::blocked_states(W) + esc;
+  return lanes > 8 && esc && lane * 4 * uint64_t(lanes) >= uint64_t(32) << 30;
+}
+
+// Residues a pass of fdp_run_sync really holds: `lanes`, or one span of 8 where, of
+// `have` bytes, the escape words fit beside 8 lanes but not beside all of them
+// (n = 22, 14 lanes: 16.4 s in one pass of single cells, 13.4 s as passes of 8 and 6).
+static int pass_lanes(int W, int lanes, uint64_t have) {
+  const uint64_t lane = (fdp::main_states(W) + fdp::blocked_states(W) + fdp::tail_escape_words(W)) * 4;
+  const bool all = lane * uint64_t(lanes) + kEscapeMargin <= have, eight = lane * 8 + kEscapeMargin <= have;
+  return may_split(W, lanes) && eight && !all ? 8 : lanes;
+}
+
 static int lanes_with_escapes(fdp_ctx *c, int W, int lanes) {
-  if (lanes <= 8 || !c->cfg.tail || whole_pass(c, W)) return lanes;
-  const size_t state = size_t(fdp::main_states(W) + fdp::blocked_states(W)) * 4, esc = fdp::tail_escape_words(W) * 4;
   size_t free_b = 0, total_b = 0;
-  if (!esc || (state + esc) * size_t(lanes) < (size_t(32) << 30) || cudaMemGetInfo(&free_b, &total_b) != cudaSuccess)
+  if (!c->cfg.tail || whole_pass(c, W) || !may_split(W, lanes) || cudaMemGetInfo(&free_b, &total_b) != cudaSuccess)
     return lanes;
-  const size_t have = free_b + pool_idle(c, c->stream) + c->cap_side + c->cap_main + c->cap_blk;
-  return (state + esc) * size_t(lanes) + kEscapeMargin > have && (state + esc) * 8 + kEscapeMargin <= have ? 8 : lanes;
+  return pass_lanes(W, lanes, free_b + pool_idle(c, c->stream) + c->cap_side + c->cap_main + c->cap_blk);
+}
+
+extern "C" int fdp_test_pass_lanes(int n, int lanes, uint64_t have_bytes) {
+  if (n < 1 || n > FDP_MAX_N || lanes < 1 || lanes > FDP_MAX_LANES) return 0;
+  return pass_lanes(n + 1, lanes, have_bytes);
+}
+
+extern "C" fdp_status fdp_test_single_cells(fdp_ctx *c, int on) {
+  if (!c) return FDP_ERR_ARGS;
+  fdp_pass_single_cells(c, on != 0);
+  return FDP_OK;
 }
 
 // Enqueue one whole residue pass on `s`: the row-0 state, the row sweeps, the

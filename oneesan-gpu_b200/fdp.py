@@ -146,6 +146,8 @@ def lib() -> ctypes.CDLL:
     L.fdp_cell_bytes.argtypes = [c_int, c_int]
     L.fdp_cell_bytes.restype = c_u64
     L.fdp_test_inject_pass_errors.argtypes = [c_int]
+    L.fdp_test_single_cells.argtypes = [c_vp, c_int]
+    L.fdp_test_pass_lanes.argtypes = [c_int, c_int, c_u64]
     _lib = L
     return L
 
@@ -283,6 +285,10 @@ class Engine:
         _check(lib().fdp_autotune(self._ctx, ctypes.byref(pr), hbm_budget_bytes, repeats, ctypes.byref(res), buf,
                                   len(buf)), "fdp_autotune")
         return _json.loads(buf.value.decode())
+
+    def single_cells(self, on: bool = True) -> None:
+        """Test hook: every cell its own launch, as where memory is short."""
+        _check(lib().fdp_test_single_cells(self._ctx, int(on)), "fdp_test_single_cells")
 
     def residues_multi(self, problems, lanes: int | None = None):
         """Several (n, moduli) problems in one captured CUDA graph; returns
