@@ -3,18 +3,22 @@
 
 Workload (default): n = 22 exact count, the 14 largest primes below 2^32 (the
 CRT prime count the checkerboard-strip bound needs at n = 22), all 14 residues
-in one batched pass (lanes = 14, one CUDA graph).  A step is one such pass:
-row-0 initialiser, 21 row sweeps of 22 cells over the HBM-resident state
-(145.6 GiB, far above L2, so no flush is needed), first-row dot product.
+in one call (one CUDA graph) of as many residues a pass as the autotuner picks
+(8 and 6 on a B200: 83.2 GiB of state, far above L2, so no flush is needed).  A
+step is one such call; each pass is a fill of the first rows, the remaining row
+sweeps of 22 cells over the HBM-resident state and the first-row dot product.
 
-value    residues/hour from the device time of the captured pass (CUDA events
+value    residues/hour from the device time of the captured call (CUDA events
          on the engine's stream), max over ranks.
 e2e      residues/hour through the public C ABI call fdp_run_sync from host
          buffers (moduli in, residues out) including graph capture.
-roofline the per-cell transition kernel: algorithmic bytes per cell
+roofline the kernel of the cells p >= 9 of a row, which a pass always launches one
+         by one and which take most of it: algorithmic bytes per cell
          (fdp_cell_bytes: 4 x words that must be read + 4 x words that can
-         change, per modulus) over the cell's CUDA-event duration (with 14
-         lanes a cell is two launches, one per lane span of at most 8).
+         change, per modulus) over the cell's CUDA-event duration (above 8 lanes
+         a cell is two launches, one per lane span of at most 8).  The cells p <=
+         8 run fused in a pass and move fewer bytes than that model counts, so a
+         whole pass has no such figure.
 
 --impl reference times the reference's own CPU counter (third_party/ggcount,
 built unmodified into oracle/_ref) on all host threads: each step is one
@@ -43,6 +47,8 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 PKG = os.path.join(ROOT, "oneesan-gpu_b200")
 sys.path.insert(0, PKG)
 sys.path.insert(0, os.path.join(ROOT, "tests"))
+
+FUSED_CELLS = 8  # cells p <= 8 of a row run as one fused pass where memory allows
 
 METRIC = "residues/hour and frontier transitions/s at n=22 on 1 B200 (batched vs plain), HBM GB/s"
 
@@ -110,8 +116,8 @@ def published_check(n: int, moduli, residues) -> dict:
 
 
 def committed_traffic(n: int, lanes: int):
-    """DRAM bytes per cell (all of the cell's lane-span launches) of the cell
-    kernel from the committed ncu summary."""
+    """DRAM bytes per cell, mean over the cells p >= 9 (all of a cell's lane-span
+    launches), from the committed ncu summary."""
     path = os.path.join(ROOT, "profiles", "cell_kernel_traffic.txt")
     if not os.path.exists(path):
         return None
@@ -385,31 +391,26 @@ def run_ours(args) -> None:
         extra["plain"] = {"value": 3600.0 / rp.stats.device_s, "unit": "residues/hour",
                           "sample": "one residue, lanes=1", "device_s": rp.stats.device_s}
 
-    # Roofline of the dominant kernel: per-cell CUDA-event times of one row sweep
-    # (a cell of more than 8 lanes is one launch per lane span of at most 8).
+    # Roofline of the dominant kernel, the cells a pass launches one by one: CUDA-event
+    # times of one row sweep (a cell of more than 8 lanes is one launch per lane span
+    # of at most 8).
     cell_ms = eng.time_cells(n, moduli, lanes, rows=args.profile_rows)
     tuning = eng.get_tuning()
     split = lanes > 8 and not tuning["split_panels"] and tuning["split_spans_min_p"] <= 1
     launches_per_cell = len(fdp.lane_spans(lanes)) if split else 1
-    tot_bytes = sum(fdp.cell_bytes(W, p) * lanes for p in range(1, W))
-    tot_ms = sum(cell_ms[1:])
+    single = range(min(FUSED_CELLS + 1, W - 1), W)
+    tot_bytes = sum(fdp.cell_bytes(W, p) * lanes for p in single)
+    tot_ms = sum(cell_ms[p] for p in single)
     achieved = tot_bytes / (tot_ms * 1e-3) / 1e9
     peaks = measured_peaks()
     traffic = committed_traffic(n, lanes)
     roof = {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
             "frac": achieved / peaks["hbm_gbs"], "traffic": traffic,
-            "kernel": "cell_kernel / cell_stream_kernel (per-cell frontier transition)",
+            "kernel": "cell_run_kernel / cell_stream_kernel (frontier transition of one cell p >= 9)",
             "peak_source": peaks["source"],
-            "alg_bytes_per_cell": tot_bytes / (W - 1), "mean_cell_ms": tot_ms / (W - 1),
-            "launches_per_cell": launches_per_cell, "row_ms": tot_ms,
+            "alg_bytes_per_cell": tot_bytes / len(single), "mean_cell_ms": tot_ms / len(single),
+            "launches_per_cell": launches_per_cell, "row_ms_of_single_cells": sum(cell_ms[1:]),
             "cell_gbs": [fdp.cell_bytes(W, p) * lanes / (cell_ms[p] * 1e-3) / 1e9 for p in range(1, W)]}
-    # The same bytes over the timed passes' device time: in a pass the two lane
-    # spans sweep as concurrent launch chains, which the per-cell timing (one
-    # span launch after the other) does not see; the row-k fill and the
-    # read-out are inside this time and not in the bytes.
-    pass_gbs = plan.alg_bytes_per_residue * k * args.steps / dev_s / 1e9
-    roof["pass_gbs"] = pass_gbs
-    roof["pass_frac"] = pass_gbs / peaks["hbm_gbs"]
     eng.close()  # frees the state before the sub-runs below
 
     transitions = plan.transitions_per_residue * k * args.steps * world
