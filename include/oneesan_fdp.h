@@ -70,8 +70,10 @@ typedef struct fdp_plan_out {
   int index_bits;                   /* 32 or 64                                   */
   uint64_t main_states;             /* H_DP[W][1]                                 */
   uint64_t blocked_states;          /* H_DP[W-1][1]                               */
-  uint64_t state_bytes;             /* 4 (M + D) lanes: the whole device footprint */
-  uint64_t scratch_bytes;           /* 0: the transition is in place              */
+  uint64_t state_bytes;             /* 4 (M + D) lanes: what a pass cannot do without */
+  uint64_t scratch_bytes;           /* 0: the transition is in place; the workspace
+                                       that fdp_run_sync takes where memory is left
+                                       is in none of these figures                */
   uint64_t table_bytes;             /* per-width index tables                     */
   uint64_t total_bytes;
   int rows;                         /* row sweeps per residue                     */
@@ -124,6 +126,16 @@ void fdp_destroy(fdp_ctx *ctx);
  * lanes = 1 is the plain one-modulus-per-launch-sequence form (the
  * reference's residue loop, GB.cu:2211-2258); lanes = k is one batched pass.
  * residues_out has k entries.
+ *
+ * Device memory: the state, 4 (M + D) lanes bytes, kept for the next call, and,
+ * where 1 GiB stays free beside it, workspace that lets the low cells of a row run
+ * as one launch (widths from 14; 0.39 words a main word and lane at width 14, 0.69
+ * at width 24).  Up to 4 GiB of workspace stay with the context until a call of it
+ * needs the memory; more is freed before the call returns.  Without room for it
+ * every cell is its own launch, with the same residues.  Where state and workspace
+ * come to 32 GiB or more and fit for 8 lanes but not for `lanes`, passes hold 8
+ * residues instead (n = 22, 14 moduli on a B200: passes of 8 and 6); fdp_plan knows
+ * no device and gives the lanes asked for.
  */
 fdp_status fdp_run_sync(fdp_ctx *ctx, const fdp_problem *problem, uint32_t *residues_out, fdp_run_stats *stats);
 
@@ -151,6 +163,12 @@ fdp_status fdp_run_multi_sync(fdp_ctx *ctx, const fdp_problem *problems, int cou
  * equal, the lanes are independent vectors under one modulus, the GROUPBATCH
  * lane semantics (src/cuda/b300/groupbatch_interleaved.cuh).
  * `stream` is a cudaStream_t (0 = the context's stream); the call is async.
+ * Device memory: tables on the first call of a width.  Besides, a window with p_hi
+ * >= 8 and p_lo = 1 (widths from 14) takes workspace as fdp_run_sync does, at most
+ * 20 GiB and only where as much again stays free, from a pool that keeps it for the
+ * next window (cudaMalloc of this process can have what lies idle there), and not
+ * on a stream under capture.  Windows with p_lo >= 2, and the window 1..1, never do:
+ * a caller that rules this out runs a row as the windows W-1..2 and 1..1.
  * `main` and `block` must be aligned to one word of the widest panel: 32
  * bytes for 8 or more lanes (an 8-lane word is one 256-bit access), 16 for
  * 4-7, 8 for 2-3 (cudaMalloc gives 256); otherwise FDP_ERR_ARGS.
@@ -230,8 +248,9 @@ fdp_status fdp_get_tuning(fdp_ctx *ctx, fdp_tuning *tuning);
  * fdp_server_start reserves hbm_budget_bytes of device memory once and starts
  * a scheduler thread.  Requests (n, moduli) queue in arrival order; a request
  * is admitted as soon as one of max_active slots and enough of the reserved
- * pool are free (its frontier, 4 (M+D) lanes bytes, stays on the device until
- * it finishes).  Later, smaller requests may pass a request that does not fit
+ * pool are free (its frontier, 4 (M+D) lanes bytes, and, unless it would not fit
+ * the whole pool with it, the workspace of fdp_run_sync stay reserved until it
+ * finishes).  Later, smaller requests may pass a request that does not fit
  * yet, unless it has waited longer than max_bypass_s.  Each admitted request
  * runs its residue pass(es) as one CUDA graph on its own stream, so admitted
  * requests overlap on the GPU and finish independently.  A request whose
@@ -253,7 +272,7 @@ typedef struct fdp_request_info {
   double latency_s;    /* submit -> completion                                   */
   double device_s;     /* CUDA-event time of the request's graph                 */
   int lanes, passes;
-  uint64_t state_bytes;
+  uint64_t state_bytes; /* pool bytes reserved: frontier, workspace, small words   */
 } fdp_request_info;
 
 typedef struct fdp_server_stats {
@@ -344,9 +363,9 @@ void fdp_transfer_map_destroy(fdp_transfer_map *map);
  * fdp_transfer_map_build; requires fixed <= p - 1 (p - 2 when paired) and
  * fixed <= 24.  fdp_factor_map_apply runs it on `groups` (<= max_groups <= 32)
  * groups at once for one modulus: the groups' values are gathered from the
- * global vectors (plain layout, one residue per state) into an arena with the
- * groups interleaved as columns, the CSR is applied column by column with one
- * reduction per output, and the results are scattered to their global ranks
+ * global vectors (plain layout, one residue per state) into an arena, one group
+ * after the other, the CSR is applied to each group with one reduction per
+ * output, and the results are scattered to their global ranks
  * in the output vectors (out_main = in_main + T x, out_block = T x on the
  * groups' rows; other rows are not written).  masks is host memory, each with
  * `occupied` set bits below bit `fixed`.  phase_ms (3 entries, may be NULL)
@@ -381,7 +400,8 @@ fdp_status fdp_reverse2_apply(fdp_ctx *ctx, int width, int p, int lanes, const u
  * framework whose own pool allocator already holds the GPU's memory (an
  * allocation would fail or break the pool's budget), or code that must not
  * take the device synchronisation cudaMalloc / cudaFree can cause.  Such a
- * caller runs the row sweeps on its own buffers (fdp_apply_cells) and then
+ * caller runs the row sweeps on its own buffers (fdp_apply_cells, each row as the
+ * windows W-1..2 and 1..1, which take no workspace) and then
  * reads the residues of its final state `d_main` (width x lanes, panel
  * layout) into `d_residues` (lanes uint32 in device memory) with this call;
  * `moduli` is host memory.  The dot product's 64-bit accumulators live in a

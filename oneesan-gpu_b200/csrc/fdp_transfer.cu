@@ -631,7 +631,7 @@ extern "C" fdp_status fdp_reverse2_apply(fdp_ctx *c, int width, int p, int lanes
   // no ranks of sources, whole panel words.  Unaligned pointers, tiny vectors,
   // streams under capture (the width's tables may have to be uploaded) and widths
   // whose tables find no memory enumerate the sources of the sources.  The line: three launches take 20 us, the
-  // enumeration 23 us for one lane of width 8 (708 words), 816 against 41 us for
+  // enumeration 23 us for one lane of width 8 (708 words), 623 against 44 us for
   // 8 lanes of width 15.
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   const bool aligned = fdp::panel_aligned(lanes, d_in_main) && fdp::panel_aligned(lanes, d_in_block) &&
@@ -668,10 +668,11 @@ extern "C" fdp_status fdp_reverse2_apply(fdp_ctx *c, int width, int p, int lanes
 // so each group is closed under the operator.  The CSR is built once, in the
 // local ranks of the representative group (the bottom `occupied` positions
 // set), and applied to up to max_groups groups at once: a gather moves each
-// group's values into an arena with the groups interleaved as columns
-// (row i of group g at i * G + g, the layout of factor_transfer_batch.cuh:13-47),
-// the apply sums every row's sources column by column with one reduction per
-// output, and a scatter writes the results back to their global ranks.
+// group's values into an arena, one group after the other (row i of group g at g *
+// rows + i, unlike the columns of factor_transfer_batch.cuh:13-47, so that a group's
+// threads read neighbouring ranks), the apply sums every row's sources with one
+// reduction per output, and a scatter writes the results to their global ranks
+// (one kernel with the apply, unless the phases are timed).
 
 namespace {
 

@@ -133,3 +133,27 @@ def test_a_second_window_in_flight_leaves_half_of_what_is_free():
         torch.cuda.empty_cache()
         assert words // 2 < taken < 3 * words // 2
         assert torch.equal(pairs[0][0], pairs[1][0]) and torch.equal(pairs[0][1], pairs[1][1])
+
+
+def test_a_row_as_two_windows_takes_no_memory():
+    import torch
+    width, mods = 20, P[:2]
+    with fdp.Engine(0) as eng:
+        g = torch.Generator(device="cuda").manual_seed(3)
+        main, blk = (torch.randint(0, 2**31 - 1, (2 * n,), dtype=torch.int32, device="cuda", generator=g)
+                     for n in (orc.main_states(width), orc.main_states(width - 1)))
+        one = main.clone(), blk.clone()
+        eng.apply_cells(width, 2, 2, mods, one[0].data_ptr(), one[1].data_ptr())  # the width's tables
+        torch.cuda.synchronize()
+        one[0].copy_(main)
+        one[1].copy_(blk)
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        eng.apply_cells(width, width - 1, 2, mods, main.data_ptr(), blk.data_ptr())
+        eng.apply_cells(width, 1, 1, mods, main.data_ptr(), blk.data_ptr())
+        assert before - torch.cuda.mem_get_info()[0] < 64 << 20  # loaded kernels
+        torch.cuda.synchronize()
+        eng.apply_cells(width, width - 1, 1, mods, one[0].data_ptr(), one[1].data_ptr())
+        torch.cuda.synchronize()
+        assert before - torch.cuda.mem_get_info()[0] > 400 << 20  # 440 MB of escape words
+        assert torch.equal(main, one[0]) and torch.equal(blk, one[1])
