@@ -318,16 +318,20 @@ static size_t pool_idle(fdp_ctx *c, cudaStream_t st) {
 
 // Device memory that one synchronous call (the context locked) takes beside its
 // state.  Up to kSideKeep bytes stay with the context for the next such call; more
-// is freed at the call's end, or no other allocator could have it: with its
-// cudaMalloc that costs 1.7 ms for 1 GiB, 10 ms for 10 GiB and 30 ms for 40 GiB, 0.7
-// % of a pass that needs so much (n = 20, 14 lanes: 1373 -> 1383 ms).
+// comes from what the windows left idle in their pool, or is freed at the call's
+// end, or no other allocator could have it: with its cudaMalloc that costs 1.7 ms
+// for 1 GiB, 10 ms for 10 GiB and 30 ms for 40 GiB, 0.7 % of a pass that needs so
+// much (n = 20, 14 lanes: 1373 -> 1383 ms), and 100 ms where the driver first has to
+// take 16 GB back from the pool.
 struct SideMemory {
   fdp_ctx *c;
   char *p = nullptr;
+  bool pooled = false;
   explicit SideMemory(fdp_ctx *ctx) : c(ctx) {}
   SideMemory(const SideMemory &) = delete;
   SideMemory &operator=(const SideMemory &) = delete;
   ~SideMemory() {
+    if (pooled) cudaFreeAsync(p, c->stream);
     if (c->cap_side > kSideKeep) drop();
   }
   void drop() {
@@ -338,8 +342,16 @@ struct SideMemory {
   }
   cudaError_t take(size_t bytes) {
     if (c->cap_side < bytes) {
-      drop();
       void *q = nullptr;
+      if (bytes > kSideKeep && pool_idle(c, c->stream) >= bytes) {
+        pooled = pool_take(c, &q, bytes, c->stream) == cudaSuccess;
+        if (pooled) {
+          p = static_cast<char *>(q);
+          return cudaSuccess;
+        }
+        cudaGetLastError();
+      }
+      drop();
       const cudaError_t e = fdp_ctx_malloc(c, &q, bytes);
       if (e != cudaSuccess) return e;
       c->d_side = static_cast<char *>(q);
