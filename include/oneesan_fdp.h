@@ -131,7 +131,8 @@ void fdp_destroy(fdp_ctx *ctx);
  * where 1 GiB stays free beside it, workspace that lets the low cells of a row run
  * as one launch (widths from 14; 0.39 words a main word and lane at width 14, 0.69
  * at width 24).  Up to 4 GiB of workspace stay with the context until a call of it
- * needs the memory; more is freed before the call returns.  Without room for it
+ * needs the memory; up to 20 GiB lie in a pool afterwards, where cudaMalloc of this
+ * process can have them; more is freed before the call returns.  Without room for it
  * every cell is its own launch, with the same residues.  Where state and workspace
  * come to 32 GiB or more and fit for 8 lanes but not for `lanes`, passes hold 8
  * residues instead (n = 22, 14 moduli on a B200: passes of 8 and 6); fdp_plan knows
@@ -165,9 +166,8 @@ fdp_status fdp_run_multi_sync(fdp_ctx *ctx, const fdp_problem *problems, int cou
  * `stream` is a cudaStream_t (0 = the context's stream); the call is async.
  * Device memory: tables on the first call of a width.  Besides, a window with p_hi
  * >= 8 and p_lo = 1 (widths from 14) takes workspace as fdp_run_sync does, at most
- * 20 GiB and only where as much again stays free, from a pool that keeps it for the
- * next window (cudaMalloc of this process can have what lies idle there), and not
- * on a stream under capture.  Windows with p_lo >= 2, and the window 1..1, never do:
+ * 20 GiB and only where as much again stays free, from the same pool, which keeps it
+ * for the next window, and not on a stream under capture.  Windows with p_lo >= 2, and the window 1..1, never do:
  * a caller that rules this out runs a row as the windows W-1..2 and 1..1.
  * `main` and `block` must be aligned to one word of the widest panel: 32
  * bytes for 8 or more lanes (an 8-lane word is one 256-bit access), 16 for

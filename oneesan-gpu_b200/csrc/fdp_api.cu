@@ -21,8 +21,8 @@ static thread_local std::string g_last_error;
 
 // Device memory a synchronous call leaves free beside its escape words.
 static constexpr size_t kEscapeMargin = size_t(1) << 30;
-// Device memory the windows' pool keeps mapped, and the most that a synchronous
-// call leaves behind, for the next one.
+// Device memory the pool keeps mapped, and the most that a synchronous call leaves
+// behind outside it, for the next one.
 static constexpr size_t kPoolKeep = size_t(20) << 30;
 static constexpr size_t kSideKeep = size_t(4) << 30;
 // Windows of a context that hold pool memory at a time.
@@ -271,7 +271,8 @@ cudaError_t fdp_ctx_malloc(fdp_ctx *c, void **p, size_t bytes) {
   return cudaMalloc(p, bytes);
 }
 
-// The pool of the windows' escape words, kept mapped up to kPoolKeep bytes.  What
+// The pool of the windows' escape words and of large side memory (SideMemory), kept
+// mapped up to kPoolKeep bytes.  What
 // lies idle in it stands in nobody's way: cudaMalloc of this process gets it from
 // the driver.
 static cudaError_t pool_take(fdp_ctx *c, void **p, size_t bytes, cudaStream_t st) {
@@ -317,12 +318,13 @@ static size_t pool_idle(fdp_ctx *c, cudaStream_t st) {
 }
 
 // Device memory that one synchronous call (the context locked) takes beside its
-// state.  Up to kSideKeep bytes stay with the context for the next such call; more
-// comes from what the windows left idle in their pool, or is freed at the call's
-// end, or no other allocator could have it: with its cudaMalloc that costs 1.7 ms
-// for 1 GiB, 10 ms for 10 GiB and 30 ms for 40 GiB, 0.7 % of a pass that needs so
-// much (n = 20, 14 lanes: 1373 -> 1383 ms), and 100 ms where the driver first has to
-// take 16 GB back from the pool.
+// state.  Up to kSideKeep bytes stay with the context for the next such call.  More
+// comes from the windows' pool, where other allocators can get it after the call:
+// the pool maps 10 GiB in 73 ms, once, and a call pays nothing for it after that
+// (cudaMalloc and cudaFree in each call: 10 ms of 1.38 s at n = 20, 14 lanes, and
+// the free waits for everything on the device, served requests too).  What exceeds
+// the pool as well is allocated and freed by the call (40 GiB 30 ms, below 0.5 % of
+// a pass that needs so much).
 struct SideMemory {
   fdp_ctx *c;
   char *p = nullptr;
@@ -331,7 +333,10 @@ struct SideMemory {
   SideMemory(const SideMemory &) = delete;
   SideMemory &operator=(const SideMemory &) = delete;
   ~SideMemory() {
-    if (pooled) cudaFreeAsync(p, c->stream);
+    if (pooled) {
+      cudaFreeAsync(p, c->stream);
+      cudaStreamSynchronize(c->stream);  // the call has waited; only now does the driver hand it on
+    }
     if (c->cap_side > kSideKeep) drop();
   }
   void drop() {
@@ -343,7 +348,7 @@ struct SideMemory {
   cudaError_t take(size_t bytes) {
     if (c->cap_side < bytes) {
       void *q = nullptr;
-      if (bytes > kSideKeep && pool_idle(c, c->stream) >= bytes) {
+      if (bytes > kSideKeep && bytes <= kPoolKeep) {
         pooled = pool_take(c, &q, bytes, c->stream) == cudaSuccess;
         if (pooled) {
           p = static_cast<char *>(q);

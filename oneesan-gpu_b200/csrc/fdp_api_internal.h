@@ -25,7 +25,7 @@ struct fdp_ctx {
   uint32_t *d_blk = nullptr;             // run_sync state, [D][lanes]
   char *d_side = nullptr;                // what a synchronous call takes beside its state
   size_t cap_main = 0, cap_blk = 0, cap_side = 0;
-  cudaMemPool_t pool = nullptr;          // escape words of fdp_apply_cells, stream-ordered
+  cudaMemPool_t pool = nullptr;          // escape words of windows, large side memory; stream-ordered
   std::vector<WindowUse> windows;        // those whose pool memory may still be in use
   unsigned long long *d_acc = nullptr;   // first-row dot accumulators
   uint32_t *d_res = nullptr;             // residues on the device
