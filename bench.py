@@ -448,7 +448,7 @@ def run_ours(args) -> None:
 
 
 def run_n20(device: int) -> dict:
-    """Config 2: n = 20, the four largest primes below 2^32, plain (one modulus
+    """n = 20, the four largest primes below 2^32, plain (one modulus
     per pass, lanes = 1) and batched (one pass of four lanes); every residue is
     checked against the reference's CPU counter (tests/golden/ggcount_residues.json)."""
     import fdp
@@ -471,7 +471,7 @@ def run_n20(device: int) -> dict:
 
 
 def run_n23(device: int, budget: int = 170 * 10**9) -> dict:
-    """Config 5: n = 23 at HBM capacity.  The largest number of the largest
+    """n = 23 at HBM capacity.  The largest number of the largest
     primes below 2^32 whose state and tables fit the budget runs as one pass;
     its residue mod 4294967291 is checked against the published value."""
     import fdp

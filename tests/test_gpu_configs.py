@@ -6,7 +6,7 @@ reference's own CPU path or to a value the reference publishes.
   (third_party/ggcount, tests/golden/ggcount_residues.json, made by
   tests/golden/gen_ggcount_residues.py);
 * n = 21: equal to the same counter for two moduli;
-* n = 22 exact count: the 14 CRT residues in one batched pass of the C++
+* n = 22 exact count: the 14 CRT residues in one batched call of the C++
   driver, every drop-one CRT subset reconstructing the same integer, and the
   residue mod 4294967291 equal to the published 1245069298
   (docs/results/groupbatch-interleaved-2026-09-05.json:1027 of the reference);
@@ -54,7 +54,7 @@ def test_n21_matches_ggcount(engine):
 
 
 def test_n22_exact_count_with_drop_one_cross_check(tmp_path):
-    # Config 3: the 14 CRT primes the path bound needs, one batched pass.
+    # The 14 CRT primes the path bound needs, one batched call.
     work = tmp_path / "n22"
     r = subprocess.run([EXACT, "22", "--work-dir", str(work), "--lanes", "14"], capture_output=True, text=True,
                        timeout=1200)
@@ -69,7 +69,7 @@ def test_n22_exact_count_with_drop_one_cross_check(tmp_path):
 
 
 def test_n23_published_residue():
-    # Config 5 at one modulus: 29.5 GiB of state, 64-bit indices.  A context of
+    # One modulus: 29.5 GiB of state, 64-bit indices.  A context of
     # its own, released at the end, so the state does not stay resident.
     with fdp.Engine(0) as eng:
         assert eng.residues(23, [4294967291], lanes=1).residues == [2762394459]

@@ -44,8 +44,9 @@ def test_published_residues(engine, n, mod, want):
 
 
 def test_lane_counts_agree(engine):
-    # Above 8 lanes a pass sweeps its two lane spans as concurrent launch
-    # chains: 9 = {0-7} + {8}, 14 = {0-7} + {8-13}, 16 = {0-7} + {8-15}.
+    # Above 8 lanes a pass has two lane spans: 9 = {0-7} + {8}, 14 = {0-7} + {8-13},
+    # 16 = {0-7} + {8-15}.  Its low cells run fused here; as single cells the spans
+    # sweep as concurrent launch chains (test_gpu_single_cells.py).
     n = 13
     mods = P[:16]
     plain = engine.residues(n, mods, lanes=1).residues
