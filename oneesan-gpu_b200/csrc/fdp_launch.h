@@ -13,7 +13,6 @@ namespace fdp {
 constexpr int kMaxLanes = 16;  // K = 1..16 residues interleaved per state
 constexpr int kCarryItems = 16;  // default states per lane of a grouped chunk with carry-over queues
 
-// Per-(width, height cap) device table blob.
 // Where the streaming cells of a span of K lanes go run by run (cell_run_kernel)
 // instead of item by item: from `from` to below `below` items per resident thread.
 // A run shares one decode and one closure scan among its items, but three CTAs per
@@ -31,6 +30,7 @@ constexpr int kCarryItems = 16;  // default states per lane of a grouped chunk w
 //   8       0.094 0.096  0.803 0.786  4.53 4.58  36.6 36.2  331   326
 // 64-bit ranks (n = 23), where a decode costs twice the instructions: 1 lane 385
 // 238, 2 428 390, 3 585 553, 4 572 590, 5 714 684; six lanes do not fit a device.
+// 7 lanes stay with items: equal at n = 21 (106.8 106.7), ahead by runs at 22 alone.
 struct RunsRange {
   uint64_t from, below;
 };
@@ -47,6 +47,7 @@ constexpr RunsRange runs_range(bool u64, int K) {
   }
 }
 
+// Per-(width, height cap) device table blob.
 struct DevTables {
   void *ptr = nullptr;
   bool u64 = false;
